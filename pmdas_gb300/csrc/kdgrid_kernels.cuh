@@ -855,49 +855,18 @@ __device__ __forceinline__ int4 rec_from_chunks(const float4* __restrict__ ch, f
     return make_int4(__float_as_int(v[0]), __float_as_int(v[1]), __float_as_int(v[2]), __float_as_int(v[3]));
 }
 
-// place, one accepted leaf (entry r of `tile`, whose prefix is `pre`, entry
-// word `e`): best candidate, append or split.  The leaf's record is read from
-// its chunks staged in shared memory at srec, or from global memory when srec
-// is null.
+// Best candidate (kdgrid.cu:332-361): of candidatesNum uniform points of the box
+// the one farthest from the leaf's samples, the first of equal ones.
 template <int D>
-__device__ __forceinline__ void place_entry(const MdasDeviceGrid& g, int tile, int r, uint2 pre, uint2 e, int N,
-                                            int L, const float4* srec = nullptr) {
-    constexpr int kMaxNodeSize = 4;
-    const int TILE = 256 * g.tileK;
-    constexpr int NB = NbLayout<D>::FLOATS;
-    (void)kMaxNodeSize;
-    const int nodeIndex = tile * TILE + (int)(e.x & 0x7ffu);
-    const int splitRankInTile = (int)((e.x >> 11) & 0x7ffu);
-    const bool split = (e.x >> 22) & 1u;
-    const int sampleCount = (int)((e.x >> 23) & 7u);
-    unsigned seed = e.y;
-    float* nb = g.nb + (size_t)nodeIndex * NB;
-    float* sc = leaf_copy<D>(g.nb, (size_t)nodeIndex);
-    float mn[D], mx[D];
-    int4 node;
-    float scv[4 * D];
-    if (srec) {
-        node = rec_from_chunks<D>(srec, mn, mx, scv);  // staged in shared memory by the warp
-    } else {
-        // the whole record (no hint: measured as fast as .L2::128B, faster than 64B or 256B)
-        node = nb_load<D>(nb, mn, mx);
-        ld_floats<4 * D>(sc, scv);
-    }
-    float samples[4][D];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int i = 0; i < D; ++i) samples[k][i] = scv[k * D + i];
-
-    // best candidate (kdgrid.cu:332-361)
-    float best[D];
+__device__ __forceinline__ void best_candidate(const float (&mn)[D], const float (&mx)[D], const float (&samples)[4][D],
+                                               int sampleCount, int candidatesNum, unsigned seed, float (&best)[D]) {
 #pragma unroll
     for (int i = 0; i < D; ++i) best[i] = 0.0f;
     float maxDistance = -1.0f;
     float diag[D];
 #pragma unroll
     for (int i = 0; i < D; ++i) diag[i] = mx[i] - mn[i];
-    for (int j = 0; j < g.candidatesNum; ++j) {
+    for (int j = 0; j < candidatesNum; ++j) {
         float rr[D];
 #pragma unroll
         for (int i = 0; i < D; ++i) rr[i] = rnd(seed);
@@ -918,7 +887,130 @@ __device__ __forceinline__ void place_entry(const MdasDeviceGrid& g, int tile, i
             for (int i = 0; i < D; ++i) best[i] = candidate[i];
         }
     }
+}
 
+// The median split of a full leaf's 5 samples (4 old in slot order, then the new
+// one): axis, position, each sample's rank along the axis and the samples of the
+// children (ranks 0 and 1: left, 2 to 4: right).
+struct SplitPlan {
+    int axis;
+    float position;
+    int rank[5];
+    int l0, l1, r0, r1, r2;
+};
+
+template <int D>
+__device__ __forceinline__ SplitPlan plan_split(const float (&mn)[D], const float (&mx)[D], const int4 node,
+                                                int sampleIndex, const float (&samples)[4][D], const float (&best)[D]) {
+    SplitPlan s;
+    // split dimension: AABB::LargestAxis, ties to the highest index (aabb.h:34-45)
+    s.axis = -1;
+    float maxExtent = -FLT_MAX;
+#pragma unroll
+    for (int i = D - 1; i >= 0; --i) {
+        const float ext = mx[i] - mn[i];
+        if (maxExtent < ext) {
+            maxExtent = ext;
+            s.axis = i;
+        }
+    }
+    // The reference bubble-sorts the 5 samples by the split coordinate
+    // (kdgrid.cu:408-417); the sort is stable, so sample k lands at rank[k] =
+    // #{m : key[m] < key[k], or key[m] == key[k] and m < k}.
+    float key[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        float v = 0.0f;
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            const float c = k < 4 ? samples[k < 4 ? k : 0][i] : best[i];
+            if (i == s.axis) v = c;
+        }
+        key[k] = v;
+    }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        int rk = 0;
+#pragma unroll
+        for (int m = 0; m < 5; ++m)
+            if (m != k) rk += (key[m] < key[k] || (key[m] == key[k] && m < k)) ? 1 : 0;
+        s.rank[k] = rk;
+    }
+    const int idx5[5] = {node.x, node.y, node.z, node.w, sampleIndex};
+    float k1 = 0.0f, k2 = 0.0f;
+    s.l0 = s.l1 = s.r0 = s.r1 = s.r2 = 0;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const int rk = s.rank[k];
+        if (rk == 1) k1 = key[k];
+        if (rk == 2) k2 = key[k];
+        if (rk == 0) s.l0 = idx5[k];
+        if (rk == 1) s.l1 = idx5[k];
+        if (rk == 2) s.r0 = idx5[k];
+        if (rk == 3) s.r1 = idx5[k];
+        if (rk == 4) s.r2 = idx5[k];
+    }
+    s.position = 0.5f * (k1 + k2);  // md = 5 >> 1 = 2
+    return s;
+}
+
+// What a split leaves besides its two records: the right child's error, count
+// and seed, and the entries of the next errors pass (the left child's error -1
+// and count 2 were written by decide).  rank: the split's rank in the pass.
+template <int D>
+__device__ __forceinline__ void store_split_lists(const MdasDeviceGrid& g, const SplitPlan& s, int nodeIndex,
+                                                  int nodeOffset, int rank, const float (&mn)[D], const float (&mx)[D]) {
+    g.errors[nodeOffset] = -1.0f;
+    g.leafCounts[nodeOffset] = 3;
+    // the children's sample lists and box volumes for the next errors pass
+    // (the volumes of the boxes in their records, by the same arithmetic)
+    float lmx[D], rmn[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+        lmx[i] = (i == s.axis) ? s.position : mx[i];
+        rmn[i] = (i == s.axis) ? s.position : mn[i];
+    }
+    g.splitL[rank] = make_int4(s.l0, s.l1, nodeIndex, __float_as_int(box_volume<D>(mn, lmx)));
+    g.splitR[rank] = make_int4(s.r0, s.r1, s.r2, __float_as_int(box_volume<D>(rmn, mx)));
+    // learned mode: the children's box extents, the first half of their
+    // raw feature rows (the errors pass writes the second)
+    if (g.featRaw) {
+        mdas_raw_store_extents<D>(g.featRaw + (size_t)rank * MDAS_RAW_FLOATS, mn, lmx);
+        mdas_raw_store_extents<D>(g.featRaw + (size_t)(g.counts->newL + rank) * MDAS_RAW_FLOATS, rmn, mx);
+    }
+    // a new slot starts without a seed: the reference's seed buffer is zeroed
+    // once at InitialSampling (kdgrid.cu:637), and a slot's first draw starts
+    // from tea<4>(slot, 0) when its seed is 0 (kdgrid.cu:323-324).  The slot
+    // stores that starting seed here instead of the 0, so that decide never
+    // computes tea<4> (a warp paid for it whenever one of its leaves was new);
+    // mdas_dump_state reports such a never-drawn seed as 0, as the reference
+    // holds it (a drawn seed is tea<4>(slot, 0) advanced by >= 1 LCG steps,
+    // which never returns to its start within the generator's 2^32 period)
+    g.seeds[nodeOffset] = tea4((unsigned)nodeOffset, 0);
+    g.dirty[rank] = nodeIndex;  // for the next errors pass
+}
+
+// place, one accepted leaf (entry r of `tile`, whose prefix is `pre`, entry
+// word `e`): best candidate, append or split, from and to global memory.
+template <int D>
+__device__ __forceinline__ void place_entry(const MdasDeviceGrid& g, int tile, int r, uint2 pre, uint2 e, int N, int L) {
+    const int TILE = 256 * g.tileK;
+    constexpr int NB = NbLayout<D>::FLOATS;
+    const int nodeIndex = tile * TILE + (int)(e.x & 0x7ffu);
+    const int splitRankInTile = (int)((e.x >> 11) & 0x7ffu);
+    const bool split = (e.x >> 22) & 1u;
+    const int sampleCount = (int)((e.x >> 23) & 7u);
+    float* nb = g.nb + (size_t)nodeIndex * NB;
+    float* sc = leaf_copy<D>(g.nb, (size_t)nodeIndex);
+    float mn[D], mx[D], scv[4 * D], samples[4][D], best[D];
+    // the whole record (no hint: measured as fast as .L2::128B, faster than 64B or 256B)
+    int4 node = nb_load<D>(nb, mn, mx);
+    ld_floats<4 * D>(sc, scv);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int i = 0; i < D; ++i) samples[k][i] = scv[k * D + i];
+    best_candidate<D>(mn, mx, samples, sampleCount, g.candidatesNum, e.y, best);
     const int sampleIndex = N + (int)pre.x + r;
     store_point<D>(g.coords + (size_t)sampleIndex * D, best);
     if (!split) {
@@ -930,102 +1022,177 @@ __device__ __forceinline__ void place_entry(const MdasDeviceGrid& g, int tile, i
         nb_set_node(nb, node);
         store_point<D>(sc + sampleCount * D, best);  // (decide wrote the new count)
     } else {
-        // split dimension: AABB::LargestAxis, ties to the highest index (aabb.h:34-45)
-        int axis = -1;
-        float maxExtent = -FLT_MAX;
-#pragma unroll
-        for (int i = D - 1; i >= 0; --i) {
-            const float ext = mx[i] - mn[i];
-            if (maxExtent < ext) {
-                maxExtent = ext;
-                axis = i;
-            }
-        }
-        // The reference bubble-sorts the 5 samples (4 old in slot order, then the
-        // new one) by the split coordinate (kdgrid.cu:408-417); the sort is stable,
-        // so sample k lands at rank[k] = #{m : key[m] < key[k], or key[m] == key[k]
-        // and m < k}.  Each sample is written straight to its ranked slot.
-        float key[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            float v = 0.0f;
-#pragma unroll
-            for (int i = 0; i < D; ++i) {
-                const float c = k < 4 ? samples[k < 4 ? k : 0][i] : best[i];
-                if (i == axis) v = c;
-            }
-            key[k] = v;
-        }
-        int rank[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            int rk = 0;
-#pragma unroll
-            for (int m = 0; m < 5; ++m)
-                if (m != k) rk += (key[m] < key[k] || (key[m] == key[k] && m < k)) ? 1 : 0;
-            rank[k] = rk;
-        }
-        const int idx5[5] = {node.x, node.y, node.z, node.w, sampleIndex};
-        float k1 = 0.0f, k2 = 0.0f;
-        int l0 = 0, l1 = 0, r0 = 0, r1 = 0, r2 = 0;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const int rk = rank[k];
-            if (rk == 1) k1 = key[k];
-            if (rk == 2) k2 = key[k];
-            if (rk == 0) l0 = idx5[k];
-            if (rk == 1) l1 = idx5[k];
-            if (rk == 2) r0 = idx5[k];
-            if (rk == 3) r1 = idx5[k];
-            if (rk == 4) r2 = idx5[k];
-        }
-        const float splitPosition = 0.5f * (k1 + k2);  // md = 5 >> 1 = 2
-        const int rank_ = (int)pre.y + splitRankInTile;
-        const int nodeOffset = L + rank_;
+        const SplitPlan s = plan_split<D>(mn, mx, node, sampleIndex, samples, best);
+        const int rank = (int)pre.y + splitRankInTile;
+        const int nodeOffset = L + rank;
         float* rnb = g.nb + (size_t)nodeOffset * NB;
         float* rsc = leaf_copy<D>(g.nb, (size_t)nodeOffset);
         // left child keeps the slot: node, mx[axis], its 2 sample coordinates;
         // right child: node, box, its 3 sample coordinates
-        nb_set_node(nb, make_int4(l0, l1, ~D, ~D));
-        nb[NbLayout<D>::BOX + D + axis] = splitPosition;
+        nb_set_node(nb, make_int4(s.l0, s.l1, ~D, ~D));
+        nb[NbLayout<D>::BOX + D + s.axis] = s.position;
         float rmn[D];
 #pragma unroll
-        for (int i = 0; i < D; ++i) rmn[i] = (i == axis) ? splitPosition : mn[i];
-        nb_store<D>(rnb, make_int4(r0, r1, r2, ~D), rmn, mx);
+        for (int i = 0; i < D; ++i) rmn[i] = (i == s.axis) ? s.position : mn[i];
+        nb_store<D>(rnb, make_int4(s.r0, s.r1, s.r2, ~D), rmn, mx);
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
-            float* dst = rank[k] < 2 ? sc + rank[k] * D : rsc + (rank[k] - 2) * D;
+            float* dst = s.rank[k] < 2 ? sc + s.rank[k] * D : rsc + (s.rank[k] - 2) * D;
             if (k < 4) store_point<D>(dst, samples[k < 4 ? k : 0]);
             else store_point<D>(dst, best);
         }
-        // (decide wrote the left child's error -1 and count 2)
-        g.errors[nodeOffset] = -1.0f;
-        g.leafCounts[nodeOffset] = 3;
-        // the children's sample lists and box volumes for the next errors pass
-        // (the volumes of the boxes written above, by the same arithmetic)
-        {
-            float lmx[D];
+        store_split_lists<D>(g, s, nodeIndex, nodeOffset, rank, mn, mx);
+    }
+}
+
+// place, the warp's accepted leaves of ranks kb .. kb + count - 1 (one per lane,
+// lanes < count active), their records staged in shared memory (lane l's at
+// slots + l * CS chunks).  Every lane of the warp calls it.
+//
+// The writes go out by whole warps: a 16-byte (or 4-byte) store instruction
+// covers consecutive chunks of few records instead of one piece of 32 records,
+// so that L1 takes a few lines per instruction and not one per lane.
+//   * The right children of a warp's splits have consecutive slots: their
+//     records are assembled in shared memory and written as one run of whole
+//     records (full sectors, the padding included).
+//   * At D = 4 a new sample's coordinates are one 16-byte store per lane, already
+//     consecutive, and an append or a left child a few; at the other dimensions
+//     (4- and 8-byte aligned points: D or D / 2 stores each) the new coordinates
+//     are staged and written as consecutive words, and appends and left children
+//     are made in the staged record, of which the changed chunks are written.
+// What bounds it at odd D when each lane writes its own pieces is the number of
+// store instructions times the lines each touches (at D = 5 about 40 scattered
+// scalar stores per split): 5-D 1920x1080 frame at 32 spp 15.96 -> 13.26 ms,
+// learned at 16 spp 8.96 -> 7.78 ms, 4-D 1024x1024 at 16 spp 2.539 -> 2.515 ms,
+// 4-D 4K at 16 spp 23.9 -> 23.4 ms (whole frames).
+template <int D>
+__device__ __forceinline__ void place_warp(const MdasDeviceGrid& g, int tile, uint2 pre, uint2 e, int N, int L, int kb,
+                                           int count, float4* slots, float* newPoints) {
+    constexpr int NB = NbLayout<D>::FLOATS, SC = NbLayout<D>::SC;
+    constexpr int C = RecChunks<D>::C, CS = RecChunks<D>::CS;
+    const int lane = threadIdx.x & 31;
+    const bool active = lane < count;
+    const int nodeIndex = tile * (256 * g.tileK) + (int)(e.x & 0x7ffu);
+    const bool split = active && ((e.x >> 22) & 1u);
+    const int sampleCount = (int)((e.x >> 23) & 7u);
+    const int sampleIndex = N + kb + lane;
+    float mn[D], mx[D], scv[4 * D], samples[4][D], best[D];
+    float* rec = reinterpret_cast<float*>(slots + lane * CS);
+    int4 node = make_int4(0, 0, 0, 0);
+    unsigned changed = 0u;  // chunks of the staged record to write back
+    if (active) {
+        node = rec_from_chunks<D>(slots + lane * CS, mn, mx, scv);
 #pragma unroll
-            for (int i = 0; i < D; ++i) lmx[i] = (i == axis) ? splitPosition : mx[i];
-            g.splitL[rank_] = make_int4(l0, l1, nodeIndex, __float_as_int(box_volume<D>(mn, lmx)));
-            g.splitR[rank_] = make_int4(r0, r1, r2, __float_as_int(box_volume<D>(rmn, mx)));
-            // learned mode: the children's box extents, the first half of their
-            // raw feature rows (the errors pass writes the second)
-            if (g.featRaw) {
-                mdas_raw_store_extents<D>(g.featRaw + (size_t)rank_ * MDAS_RAW_FLOATS, mn, lmx);
-                mdas_raw_store_extents<D>(g.featRaw + (size_t)(g.counts->newL + rank_) * MDAS_RAW_FLOATS, rmn, mx);
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int i = 0; i < D; ++i) samples[k][i] = scv[k * D + i];
+        best_candidate<D>(mn, mx, samples, sampleCount, g.candidatesNum, e.y, best);
+        if constexpr (D == 4) {
+            store_point<D>(g.coords + (size_t)sampleIndex * D, best);
+        } else {
+#pragma unroll
+            for (int i = 0; i < D; ++i) newPoints[lane * D + i] = best[i];
+        }
+        if (!split) {
+            // room left: append the index (and its coordinates), the error stays as it was
+            if constexpr (D == 4) {
+                if (sampleCount == 0) node.x = sampleIndex;
+                else if (sampleCount == 1) node.y = sampleIndex;
+                else if (sampleCount == 2) node.z = sampleIndex;
+                else node.w = sampleIndex;
+                float* nb = g.nb + (size_t)nodeIndex * NB;
+                nb_set_node(nb, node);
+                store_point<D>(nb + SC + sampleCount * D, best);  // (decide wrote the new count)
+            } else {
+                rec[sampleCount] = __int_as_float(sampleIndex);
+                const int at = SC + sampleCount * D;
+#pragma unroll
+                for (int i = 0; i < D; ++i) rec[at + i] = best[i];
+                const int c0 = at >> 2, c1 = (at + D - 1) >> 2;
+                changed = 1u | ((2u << c1) - (1u << c0));
             }
         }
-        // a new slot starts without a seed: the reference's seed buffer is zeroed
-        // once at InitialSampling (kdgrid.cu:637), and a slot's first draw starts
-        // from tea<4>(slot, 0) when its seed is 0 (kdgrid.cu:323-324).  The slot
-        // stores that starting seed here instead of the 0, so that decide never
-        // computes tea<4> (a warp paid for it whenever one of its leaves was new);
-        // mdas_dump_state reports such a never-drawn seed as 0, as the reference
-        // holds it (a drawn seed is tea<4>(slot, 0) advanced by >= 1 LCG steps,
-        // which never returns to its start within the generator's 2^32 period)
-        g.seeds[nodeOffset] = tea4((unsigned)nodeOffset, 0);
-        g.dirty[rank_] = nodeIndex;  // for the next errors pass
+    }
+    SplitPlan s;
+    if (split) {
+        s = plan_split<D>(mn, mx, node, sampleIndex, samples, best);
+        // left child keeps the slot: node, mx[axis], its 2 sample coordinates
+        if constexpr (D == 4) {
+            float* nb = g.nb + (size_t)nodeIndex * NB;
+            nb_set_node(nb, make_int4(s.l0, s.l1, ~D, ~D));
+            nb[NbLayout<D>::BOX + D + s.axis] = s.position;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                if (s.rank[k] >= 2) continue;
+                if (k < 4) store_point<D>(nb + SC + s.rank[k] * D, samples[k < 4 ? k : 0]);
+                else store_point<D>(nb + SC + s.rank[k] * D, best);
+            }
+        } else {
+            reinterpret_cast<int4*>(rec)[0] = make_int4(s.l0, s.l1, ~D, ~D);
+            rec[NbLayout<D>::BOX + D + s.axis] = s.position;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                if (s.rank[k] >= 2) continue;
+#pragma unroll
+                for (int i = 0; i < D; ++i)
+                    rec[SC + s.rank[k] * D + i] = k < 4 ? samples[k < 4 ? k : 0][i] : best[i];
+            }
+            constexpr int c1 = (SC + 2 * D - 1) >> 2;
+            changed = 1u | (1u << ((NbLayout<D>::BOX + D + s.axis) >> 2)) | ((2u << c1) - (1u << (SC >> 2)));
+        }
+    }
+    if constexpr (D != 4) {
+        __syncwarp();
+        float* dst = g.coords + (size_t)(N + kb) * D;
+        for (int t = lane; t < count * D; t += 32) dst[t] = newPoints[t];
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            const int t = q * 32 + lane;
+            const int r = t / C, c = t - r * C;
+            const unsigned m = __shfl_sync(0xffffffffu, changed, r);
+            const int leaf = __shfl_sync(0xffffffffu, nodeIndex, r);
+            if ((m >> c) & 1u)
+                *reinterpret_cast<float4*>(g.nb + (size_t)leaf * NB + 4 * c) = slots[r * CS + c];
+        }
+    }
+    const unsigned splits = __ballot_sync(0xffffffffu, split);
+    if (splits) {
+        __syncwarp();  // every lane's record is read: the slots take the right children
+        const int rank = (int)pre.y + (int)((e.x >> 11) & 0x7ffu);
+        const int rank0 = __shfl_sync(0xffffffffu, rank, __ffs(splits) - 1);
+        if (split) {
+            float4* out = slots + __popc(splits & ((1u << lane) - 1u)) * CS;
+            float v[SC];
+            v[0] = __int_as_float(s.r0);
+            v[1] = __int_as_float(s.r1);
+            v[2] = __int_as_float(s.r2);
+            v[3] = __int_as_float(~D);
+#pragma unroll
+            for (int i = 0; i < D; ++i) {
+                v[4 + i] = (i == s.axis) ? s.position : mn[i];
+                v[4 + D + i] = mx[i];
+            }
+#pragma unroll
+            for (int i = 4 + 2 * D; i < SC; ++i) v[i] = 0.0f;
+#pragma unroll
+            for (int c = 0; c < SC / 4; ++c) out[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+            float* pts = reinterpret_cast<float*>(out) + SC;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                if (s.rank[k] < 2) continue;
+                float* p = pts + (s.rank[k] - 2) * D;
+                if (k < 4) store_point<D>(p, samples[k < 4 ? k : 0]);
+                else store_point<D>(p, best);
+            }
+            store_split_lists<D>(g, s, nodeIndex, L + rank, rank, mn, mx);
+        }
+        __syncwarp();
+        float4* dst = reinterpret_cast<float4*>(g.nb + (size_t)(L + rank0) * NB);
+        const int chunks = __popc(splits) * (NB / 4);
+        for (int t = lane; t < chunks; t += 32) {
+            const int r = t / (NB / 4), c = t - r * (NB / 4);
+            dst[t] = c < C ? slots[r * CS + c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
     }
 }
 
@@ -1051,15 +1218,25 @@ template <int D>
 __device__ __forceinline__ void stage_records(const float* __restrict__ nb, int leaf, float4* srec) {
     constexpr int C = RecChunks<D>::C, CS = RecChunks<D>::CS, NB = NbLayout<D>::FLOATS;
     const int lane = threadIdx.x & 31;
-    // each record takes P lanes (P: C rounded up to a power of two), chunk = lane % P
-    constexpr int P = C <= 8 ? 8 : 16;
-    constexpr int RPQ = 32 / P;  // records per copy instruction
-    const int c = lane & (P - 1), r0 = lane / P;
+    if constexpr (C == 7) {
+        // each record takes 8 lanes, chunk = lane % 8
+        const int c = lane & 7, r0 = lane >> 3;
 #pragma unroll
-    for (int q = 0; q < P; ++q) {
-        const int rr = q * RPQ + r0;
-        const int src = __shfl_sync(0xffffffffu, leaf, rr);
-        if (c < C && src >= 0) cp_async16(srec + rr * CS + c, nb + (size_t)src * NB + 4 * c);
+        for (int q = 0; q < 8; ++q) {
+            const int rr = q * 4 + r0;
+            const int src = __shfl_sync(0xffffffffu, leaf, rr);
+            if (c < C && src >= 0) cp_async16(srec + rr * CS + c, nb + (size_t)src * NB + 4 * c);
+        }
+    } else {
+        // consecutive chunks of the warp's records on consecutive lanes: C copies
+        // (at C = 9 or 10, a power of two of lanes per record would take 16)
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            const int t = q * 32 + lane;
+            const int rr = t / C, c = t - rr * C;
+            const int src = __shfl_sync(0xffffffffu, leaf, rr);
+            if (src >= 0) cp_async16(srec + rr * CS + c, nb + (size_t)src * NB + 4 * c);
+        }
     }
 }
 
@@ -1113,6 +1290,7 @@ template <int D>
 __global__ void __launch_bounds__(256, D >= 5 ? 2 : 3) k_adaptive_place(MdasDeviceGrid g) {
     constexpr int CS = RecChunks<D>::CS;
     __shared__ __align__(16) float4 s_rec[2][8][32 * CS];
+    __shared__ float s_new[D == 4 ? 1 : 8][D == 4 ? 1 : 32 * D];  // the warps' new points (place_warp)
     pdl_wait();
     const int N = g.ctl->N0;
     const int L = g.ctl->L0;
@@ -1150,9 +1328,8 @@ __global__ void __launch_bounds__(256, D >= 5 ? 2 : 3) k_adaptive_place(MdasDevi
             cp_async_wait_group<0>();
         }
         __syncwarp();
-        const int k = kb + lane;
-        if (k < accepted)
-            place_entry<D>(g, tile0, k - (int)pre0.x, pre0, e0, N, L, s_rec[buf][warp] + lane * CS);
+        place_warp<D>(g, tile0, pre0, e0, N, L, kb, min(32, accepted - kb), s_rec[buf][warp],
+                      s_new[D == 4 ? 0 : warp]);
         __syncwarp();  // the buffer is refilled two iterations on
         if (!more) break;
         e0 = e1;
