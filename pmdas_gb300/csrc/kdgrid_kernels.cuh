@@ -803,29 +803,6 @@ __global__ void __launch_bounds__(1024) k_adaptive_scan(MdasDeviceGrid g) {
     scan_image(g, s_sel, s_split);
 }
 
-// Where entry k of the pass's accepted list (its new sample is N + k) lies:
-// its tile (found from the first tile of its 256-entry chunk), the tile's
-// prefix, its rank in the tile and its entry word.
-struct PlaceLoc {
-    int tile, r;
-    uint2 pre, e;
-};
-
-__device__ __forceinline__ PlaceLoc place_locate(const MdasDeviceGrid& g, int k, int ntiles) {
-    PlaceLoc p;
-    p.tile = g.chunkTile[k >> 8];
-    p.pre = g.tilePrefix[p.tile];
-    while (p.tile + 1 < ntiles) {
-        const uint2 next = g.tilePrefix[p.tile + 1];
-        if ((int)next.x > k) break;
-        ++p.tile;
-        p.pre = next;
-    }
-    p.r = k - (int)p.pre.x;
-    p.e = g.accepted[(size_t)p.tile * (256 * g.tileK) + p.r];
-    return p;
-}
-
 // 16-byte chunks of a leaf record that the adaptive pass reads (node, box, padding, private copy)
 template <int D>
 struct RecChunks {
@@ -990,61 +967,6 @@ __device__ __forceinline__ void store_split_lists(const MdasDeviceGrid& g, const
     g.dirty[rank] = nodeIndex;  // for the next errors pass
 }
 
-// place, one accepted leaf (entry r of `tile`, whose prefix is `pre`, entry
-// word `e`): best candidate, append or split, from and to global memory.
-template <int D>
-__device__ __forceinline__ void place_entry(const MdasDeviceGrid& g, int tile, int r, uint2 pre, uint2 e, int N, int L) {
-    const int TILE = 256 * g.tileK;
-    constexpr int NB = NbLayout<D>::FLOATS;
-    const int nodeIndex = tile * TILE + (int)(e.x & 0x7ffu);
-    const int splitRankInTile = (int)((e.x >> 11) & 0x7ffu);
-    const bool split = (e.x >> 22) & 1u;
-    const int sampleCount = (int)((e.x >> 23) & 7u);
-    float* nb = g.nb + (size_t)nodeIndex * NB;
-    float* sc = leaf_copy<D>(g.nb, (size_t)nodeIndex);
-    float mn[D], mx[D], scv[4 * D], samples[4][D], best[D];
-    // the whole record (no hint: measured as fast as .L2::128B, faster than 64B or 256B)
-    int4 node = nb_load<D>(nb, mn, mx);
-    ld_floats<4 * D>(sc, scv);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int i = 0; i < D; ++i) samples[k][i] = scv[k * D + i];
-    best_candidate<D>(mn, mx, samples, sampleCount, g.candidatesNum, e.y, best);
-    const int sampleIndex = N + (int)pre.x + r;
-    store_point<D>(g.coords + (size_t)sampleIndex * D, best);
-    if (!split) {
-        // room left: append the index (and its coordinates), the error stays as it was
-        if (sampleCount == 0) node.x = sampleIndex;
-        else if (sampleCount == 1) node.y = sampleIndex;
-        else if (sampleCount == 2) node.z = sampleIndex;
-        else node.w = sampleIndex;
-        nb_set_node(nb, node);
-        store_point<D>(sc + sampleCount * D, best);  // (decide wrote the new count)
-    } else {
-        const SplitPlan s = plan_split<D>(mn, mx, node, sampleIndex, samples, best);
-        const int rank = (int)pre.y + splitRankInTile;
-        const int nodeOffset = L + rank;
-        float* rnb = g.nb + (size_t)nodeOffset * NB;
-        float* rsc = leaf_copy<D>(g.nb, (size_t)nodeOffset);
-        // left child keeps the slot: node, mx[axis], its 2 sample coordinates;
-        // right child: node, box, its 3 sample coordinates
-        nb_set_node(nb, make_int4(s.l0, s.l1, ~D, ~D));
-        nb[NbLayout<D>::BOX + D + s.axis] = s.position;
-        float rmn[D];
-#pragma unroll
-        for (int i = 0; i < D; ++i) rmn[i] = (i == s.axis) ? s.position : mn[i];
-        nb_store<D>(rnb, make_int4(s.r0, s.r1, s.r2, ~D), rmn, mx);
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            float* dst = s.rank[k] < 2 ? sc + s.rank[k] * D : rsc + (s.rank[k] - 2) * D;
-            if (k < 4) store_point<D>(dst, samples[k < 4 ? k : 0]);
-            else store_point<D>(dst, best);
-        }
-        store_split_lists<D>(g, s, nodeIndex, nodeOffset, rank, mn, mx);
-    }
-}
-
 // place, the warp's accepted leaves of ranks kb .. kb + count - 1 (one per lane,
 // lanes < count active), their records staged in shared memory (lane l's at
 // slots + l * CS chunks).  Every lane of the warp calls it.
@@ -1194,13 +1116,6 @@ __device__ __forceinline__ void place_warp(const MdasDeviceGrid& g, int tile, ui
             dst[t] = c < C ? slots[r * CS + c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
-}
-
-template <int D>
-__device__ __forceinline__ void place_rank(const MdasDeviceGrid& g, int k, int N, int L) {
-    const int ntiles = (L + 256 * g.tileK - 1) / (256 * g.tileK);
-    const PlaceLoc p = place_locate(g, k, ntiles);
-    place_entry<D>(g, p.tile, p.r, p.pre, p.e, N, L);
 }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
