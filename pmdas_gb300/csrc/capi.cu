@@ -1081,6 +1081,9 @@ struct mdas_batch {
     MdasBatchScene* d_scenes = nullptr;
     bool anyActive = false;
     cudaStream_t stream = nullptr, captureStream = nullptr, bodyStream = nullptr;
+    // the branches of a pass: one per dimension after the first (enqueue_batch_body)
+    cudaStream_t groupStream[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t forkEvent = nullptr, joinEvent[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaGraphExec_t exec = nullptr;
     int tune[4] = {4, 4, 4, 8};  // persistent CTAs per SM: errors, decide, place, integrate/integrand
     int tileK = MDAS_LEAVES_PER_THREAD;  // leaves per thread of decide (tiles of 256 * tileK leaves)
@@ -1115,25 +1118,33 @@ cudaError_t enqueue_batch_body(mdas_batch* b, cudaGraphConditionalHandle handle,
     const int gInt = b->numSMs * b->tune[3];
     // (the accumulators of this pass were cleared by the last pass's scan, or
     // when the counters were set)
+    // The dimensions' passes do not depend on one another: each dimension's chain
+    // of launches is a branch of its own, so that a short kernel of one fills the
+    // SMs that the last CTAs of another's leave (12 images of D = 3 and 4: 46.0 ->
+    // 43.1 ms).  The first dimension present stays on s.
     cudaError_t e = cudaSuccess;
-    for (const auto& gr : b->groups)
-        if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_errors, b->d_imgs + gr.offset, gr.count, gr.D, gErr, s);
-    if (e == cudaSuccess && b->anyLearned) {
-        // learned images: priorities of the leaves whose error was recomputed, then the judge
-        e = MDAS_ARITH_CALL(b, batch_reset, b->d_imgs, b->n, 2, s);
-        for (const auto& gr : b->groups)
-            if (e == cudaSuccess) e = mdas_mlp::batch_predict(b->d_imgs + gr.offset, gr.count, gr.D, b->status, s);
-        if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_learned_judge, b->d_imgs, b->n, b->numSMs * 4, s);
-    }
-    for (const auto& gr : b->groups)
+    if (b->groups.size() > 1) e = cudaEventRecord(b->forkEvent, s);
+    for (size_t k = 0; k < b->groups.size() && e == cudaSuccess; ++k) {
+        const auto& gr = b->groups[k];
+        const MdasBatchImage* imgs = b->d_imgs + gr.offset;
+        const cudaStream_t gs = k == 0 ? s : b->groupStream[k];
+        if (k > 0) e = cudaStreamWaitEvent(gs, b->forkEvent, 0);
+        if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_errors, imgs, gr.count, gr.D, gErr, gs);
+        if (e == cudaSuccess && b->anyLearned) {
+            // learned images: priorities of the leaves whose error was recomputed, then the judge
+            e = MDAS_ARITH_CALL(b, batch_reset, imgs, gr.count, 2, gs);
+            if (e == cudaSuccess) e = mdas_mlp::batch_predict(imgs, gr.count, gr.D, b->status, gs);
+            if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_learned_judge, imgs, gr.count, b->numSMs * 4, gs);
+        }
         if (e == cudaSuccess)
-            e = MDAS_ARITH_CALL(b, batch_decide, b->d_imgs + gr.offset, gr.count, gr.D, b->tileK, b->anyLearned, gDec,
-                                s);
-    if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_scan, b->d_imgs, b->n, s);
-    for (const auto& gr : b->groups)
-        if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_place, b->d_imgs + gr.offset, gr.count, gr.D, gPl, s);
-    for (const auto& gr : b->groups)
-        if (e == cudaSuccess) e = mdas_launch_evaluate_batch(b->d_scenes + gr.offset, gr.count, gr.D, 0, gInt, s);
+            e = MDAS_ARITH_CALL(b, batch_decide, imgs, gr.count, gr.D, b->tileK, b->anyLearned, gDec, gs);
+        if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_scan, imgs, gr.count, gs);
+        if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_place, imgs, gr.count, gr.D, gPl, gs);
+        if (e == cudaSuccess)
+            e = mdas_launch_evaluate_batch(b->d_scenes + gr.offset, gr.count, gr.D, 0, gInt, gs);
+        if (k > 0 && e == cudaSuccess) e = cudaEventRecord(b->joinEvent[k], gs);
+    }
+    for (size_t k = 1; k < b->groups.size() && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(s, b->joinEvent[k], 0);
     if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_condition, b->d_imgs, b->n, handle, kMaxGraphPasses, anyOut, s);
     return e;
 }
@@ -1206,6 +1217,11 @@ void free_batch(mdas_batch* b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->captureStream) cudaStreamDestroy(b->captureStream);
     if (b->bodyStream) cudaStreamDestroy(b->bodyStream);
+    for (int k = 0; k < 4; ++k) {
+        if (b->groupStream[k]) cudaStreamDestroy(b->groupStream[k]);
+        if (b->joinEvent[k]) cudaEventDestroy(b->joinEvent[k]);
+    }
+    if (b->forkEvent) cudaEventDestroy(b->forkEvent);
     cudaFree(b->d_imgs);
     cudaFree(b->d_scenes);
     cudaFree(b->status);
@@ -1289,7 +1305,11 @@ int mdas_batch_create(mdas_batch** out, int n, mdas_grid* const* grids, mdas_sce
               cudaMalloc(&b->status, sizeof(unsigned)) == cudaSuccess &&
               cudaMemset(b->status, 0, sizeof(unsigned)) == cudaSuccess &&
               cudaStreamCreateWithFlags(&b->captureStream, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaStreamCreateWithFlags(&b->bodyStream, cudaStreamNonBlocking) == cudaSuccess;
+              cudaStreamCreateWithFlags(&b->bodyStream, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaEventCreateWithFlags(&b->forkEvent, cudaEventDisableTiming) == cudaSuccess;
+    for (size_t k = 1; k < b->groups.size() && ok; ++k)
+        ok = cudaStreamCreateWithFlags(&b->groupStream[k], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&b->joinEvent[k], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         free_batch(b);
