@@ -863,9 +863,7 @@ int mdas_scene_reference_image(mdas_scene* s, int width, int height, int spp, ui
     int nsm = 1, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t want = ((int64_t)width * height + 255) / 256;
-    const int grid = (int)(want < (int64_t)nsm * 16 ? want : (int64_t)nsm * 16);
-    return status_of(mdas_launch_reference_image(s->desc, s->d_prims, width, height, strata, seed, out, grid,
+    return status_of(mdas_launch_reference_image(s->desc, s->d_prims, s->d_cull, width, height, strata, seed, out, nsm,
                                                  (cudaStream_t)stream));
 }
 
@@ -1932,7 +1930,7 @@ int mdas_leaf_true_errors(mdas_grid* g, mdas_scene* s, int samplesPerLeaf, uint6
     if (!g->initialized) return MDAS_ERR_STATE;
     int rc = scene_upload(s, g->stream);
     if (rc) return rc;
-    cudaError_t e = mdas_launch_leaf_true_errors(s->desc, s->d_prims, g->dg, leaves, leaves ? count : g->L,
+    cudaError_t e = mdas_launch_leaf_true_errors(s->desc, s->d_prims, s->d_cull, g->dg, leaves, leaves ? count : g->L,
                                                  samplesPerLeaf, seed, errors, g->stream);
     g->launches += 1;
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);

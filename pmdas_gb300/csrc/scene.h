@@ -26,12 +26,14 @@ cudaError_t mdas_launch_evaluate(const MdasScene& sc, const float* d_prims, cons
                                  float* values, int dim, const MdasCounts* counts, int offset, int count, int grid,
                                  cudaStream_t s);
 
-cudaError_t mdas_launch_leaf_true_errors(const MdasScene& sc, const float* d_prims, const MdasDeviceGrid& g,
-                                         const int* leaves, int L, int samples, unsigned long long seed, float* out,
-                                         cudaStream_t s);
+cudaError_t mdas_launch_leaf_true_errors(const MdasScene& sc, const float* d_prims, const unsigned* cull,
+                                         const MdasDeviceGrid& g, const int* leaves, int L, int samples,
+                                         unsigned long long seed, float* out, cudaStream_t s);
 
-cudaError_t mdas_launch_reference_image(const MdasScene& sc, const float* d_prims, int width, int height, int strata,
-                                        unsigned long long seed, double* out, int grid, cudaStream_t s);
+// sms: SMs of the device.
+cudaError_t mdas_launch_reference_image(const MdasScene& sc, const float* d_prims, const unsigned* cull, int width,
+                                        int height, int strata, unsigned long long seed, double* out, int sms,
+                                        cudaStream_t s);
 
 int mdas_generate_scene(int kind, uint64_t seed, int count, float scaleX, float scaleY, int width, int height,
                         MdasScene* sc, std::vector<float>* prims);
