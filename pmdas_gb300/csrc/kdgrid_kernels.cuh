@@ -183,16 +183,21 @@ __device__ __forceinline__ float box_volume(const float (&mn)[D], const float (&
     return res;
 }
 
-// PointN::Distance (point.h:172-182)
+// PointN::Distance (point.h:172-182), and its square
 template <int D>
-__device__ __forceinline__ float distance(const float (&a)[D], const float (&b)[D]) {
+__device__ __forceinline__ float distance2(const float (&a)[D], const float (&b)[D]) {
     float result = 0.0f;
 #pragma unroll
     for (int i = 0; i < D; ++i) {
         const float d = a[i] - b[i];
         result += d * d;
     }
-    return sqrtf(result);
+    return result;
+}
+
+template <int D>
+__device__ __forceinline__ float distance(const float (&a)[D], const float (&b)[D]) {
+    return sqrtf(distance2<D>(a, b));
 }
 
 __device__ __forceinline__ int node_count(const int4 n) {
@@ -832,6 +837,33 @@ __device__ __forceinline__ int4 rec_from_chunks(const float4* __restrict__ ch, f
     return make_int4(__float_as_int(v[0]), __float_as_int(v[1]), __float_as_int(v[2]), __float_as_int(v[3]));
 }
 
+// The smallest distance of a candidate to the leaf's first sampleCount samples
+// (FLT_MAX without any), kdgrid.cu:341-351.  All four distances are computed and
+// those of empty slots dropped: a branch per slot cost more than the distance.
+template <int D>
+__device__ __forceinline__ float min_distance(const float (&candidate)[D], const float (&samples)[4][D],
+                                              int sampleCount) {
+#ifdef MDAS_REFERENCE_ARITH
+    float m = FLT_MAX;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float d = distance<D>(candidate, samples[k]);
+        m = fminf(m, k < sampleCount ? d : FLT_MAX);
+    }
+    return m;
+#else
+    // the correctly rounded square root is monotonic: one root, of the smallest
+    // square (the approximate one is not, so that build takes every root)
+    float m2 = __int_as_float(0x7f800000);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float d2 = distance2<D>(candidate, samples[k]);
+        m2 = fminf(m2, k < sampleCount ? d2 : m2);
+    }
+    return fminf(FLT_MAX, sqrtf(m2));
+#endif
+}
+
 // Best candidate (kdgrid.cu:332-361): of candidatesNum uniform points of the box
 // the one farthest from the leaf's samples, the first of equal ones.
 template <int D>
@@ -850,19 +882,11 @@ __device__ __forceinline__ void best_candidate(const float (&mn)[D], const float
         float candidate[D];
 #pragma unroll
         for (int i = 0; i < D; ++i) candidate[i] = mn[i] + rr[i] * diag[i];
-        float minDistance = FLT_MAX;
+        const float minDistance = min_distance<D>(candidate, samples, sampleCount);
+        const bool better = maxDistance < minDistance;
+        maxDistance = better ? minDistance : maxDistance;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (k < sampleCount) {
-                const float distance_k = distance<D>(candidate, samples[k]);
-                if (minDistance > distance_k) minDistance = distance_k;
-            }
-        }
-        if (maxDistance < minDistance) {
-            maxDistance = minDistance;
-#pragma unroll
-            for (int i = 0; i < D; ++i) best[i] = candidate[i];
-        }
+        for (int i = 0; i < D; ++i) best[i] = better ? candidate[i] : best[i];
     }
 }
 
@@ -910,7 +934,7 @@ __device__ __forceinline__ SplitPlan plan_split(const float (&mn)[D], const floa
         int rk = 0;
 #pragma unroll
         for (int m = 0; m < 5; ++m)
-            if (m != k) rk += (key[m] < key[k] || (key[m] == key[k] && m < k)) ? 1 : 0;
+            if (m != k) rk += (m < k ? key[m] <= key[k] : key[m] < key[k]) ? 1 : 0;
         s.rank[k] = rk;
     }
     const int idx5[5] = {node.x, node.y, node.z, node.w, sampleIndex};
