@@ -327,8 +327,7 @@ __device__ __forceinline__ float node_error(const MdasDeviceGrid& g, const int4 
     for (int i = 0; i < 4; ++i) {
         const int idx = node_get(node, i);
         if (idx >= 0) {
-            const float* v = g.values + 3 * (size_t)idx;
-            loc[i] = make_float3(__ldg(v), __ldg(v + 1), __ldg(v + 2));
+            loc[i] = ld_value64(g.values, idx);
             avg.x += loc[i].x;
             avg.y += loc[i].y;
             avg.z += loc[i].z;
@@ -1300,10 +1299,10 @@ __device__ __forceinline__ void integrate_leaf(const MdasDeviceGrid& g, const in
     for (int i = 0; i < 4; ++i) {
         const int idx = node_get(node, i);
         if (idx >= 0) {
-            const float* v = g.values + 3 * (size_t)idx;
-            sampleValue.x += __ldg(v);
-            sampleValue.y += __ldg(v + 1);
-            sampleValue.z += __ldg(v + 2);
+            const float3 v = ld_value64(g.values, idx);
+            sampleValue.x += v.x;
+            sampleValue.y += v.y;
+            sampleValue.z += v.z;
             sampleCount++;
         }
     }

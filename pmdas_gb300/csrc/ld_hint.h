@@ -26,6 +26,15 @@ __device__ __forceinline__ float4 ld4_hint(const float* p) {
     return v;
 }
 
+__device__ __forceinline__ float3 ld_value64(const float* __restrict__ values, int idx) {
+    const float* p = values + 3 * (size_t)idx;
+    float3 v;
+    asm ("ld.global.L2::64B.f32 %0, [%1];" : "=f"(v.x) : "l"(p));
+    asm ("ld.global.L2::64B.f32 %0, [%1];" : "=f"(v.y) : "l"(p + 1));
+    asm ("ld.global.L2::64B.f32 %0, [%1];" : "=f"(v.z) : "l"(p + 2));
+    return v;
+}
+
 // The first NF floats of a 16-byte aligned record (rounded up to 16-byte
 // chunks: the record must extend that far) with the 64-byte hint.
 template <int NF>
