@@ -17,6 +17,8 @@
 // and the weight gradients dW2 = dZ2^T H1, dW1 = dZ1^T X as one GEMM per tile
 // (M 128, N 80, K 128 over the tile's rows) accumulated in tensor memory over
 // all tiles of a persistent CTA, added to the global gradient once per CTA.
+// That GEMM contracts over the rows, so it reads the row tiles [dZ2 | dZ1] and
+// [H1 | X] as they lie, as MN-major operands: nothing is transposed.
 #include "mlp.h"
 #include "leaf_raw.h"
 #include "ld_hint.h"
@@ -36,8 +38,11 @@ constexpr uint32_t kTmemCols = 64;
 constexpr int kWaitLimit = 1 << 20;
 
 // shared-memory map (bytes from the 1024-aligned base)
-constexpr int SM_X = 0;          // 128 x 16 BF16, core matrices, 2 K-blocks per row group
-constexpr int SM_H = 4096;       // 128 x 64 BF16, 8 K-blocks per row group
+// 128 x 80 BF16, [H1 | X]: 10 K-blocks per row group (H1 in blocks 0-7, the
+// features X in 8 and 9)
+constexpr int SM_HX = 0;
+constexpr int kHxBlocks = (kH + kIn) / 8;
+constexpr int SM_X = SM_HX + (kH / 8) * 128;  // its X part
 constexpr int SM_W1 = 20480;     // 64 x 16 BF16
 constexpr int SM_W2 = 22528;     // 64 x 64 BF16 (B of layer 2: n = output, k = input)
 constexpr int SM_W2T = 30720;    // 64 x 64 BF16 (B of dH1: n = input, k = output)
@@ -48,18 +53,18 @@ constexpr int SM_BAR = 39744;    // mbarrier (8 B), TMEM address slot (4 B)
 constexpr int SM_BIAS = 39808;
 constexpr int SM_FWD = SM_BIAS + 2 * 16 * 128;  // end of what the forward needs
 // training only
-constexpr int SM_Z2F = 44032;                    // dZ2, FP32 [128][65]
-constexpr int SM_D = SM_Z2F + kRows * 65 * 4;    // dZ2, BF16 core matrices (A of dH1)
-constexpr int SM_Z1F = SM_D + kRows * kH * 2;    // dZ1, FP32 [128][65]
-constexpr int SM_G = SM_Z1F + kRows * 65 * 4;    // per-CTA gradient, FP32 [MDAS_MLP_PARAMS]
-constexpr int SM_RED = SM_G + ((MDAS_MLP_PARAMS * 4 + 127) / 128) * 128;  // [3][4 warps][64] partial sums
-constexpr int SM_TRAIN = SM_RED + 3 * 4 * kH * 4;
+constexpr int SM_G = 44032;                      // 128 x 128 BF16, [dZ2 | dZ1]: 16 K-blocks per row group
+constexpr int kGBlocks = 2 * kH / 8;
+constexpr int SM_RED = SM_G + kRows * 2 * kH * 2;  // [3][4 warps][64] partial sums
+constexpr int SM_VG = SM_RED + 3 * 4 * kH * 4;     // the CTA's gradients of w3, b2, b1 (64 floats each), b3
+constexpr int SM_TRAIN = SM_VG + (3 * kH + 4) * 4;
 constexpr int kFwdSmem = SM_FWD + 1024;          // (+ alignment of the base) <= 5 CTAs x 64 TMEM columns per SM
-constexpr int kTrainSmem = SM_TRAIN + 1024;
+constexpr int kTrainSmem = SM_TRAIN + 1024;      // two CTAs per SM (79 KB each, 256 TMEM columns each)
 
+static_assert(kRows * (kH + kIn) * 2 == SM_W1, "map");
 static_assert(SM_W2T + kH * kH * 2 == SM_VEC, "map");
 static_assert(SM_VEC + (3 * kH + 4) * 4 <= SM_BAR, "map");
-static_assert(SM_FWD <= SM_Z2F && SM_BIAS >= SM_BAR + 16 && SM_BIAS % 128 == 0, "map");
+static_assert(SM_FWD <= SM_G && SM_BIAS >= SM_BAR + 16 && SM_BIAS % 128 == 0, "map");
 
 // ---- PTX wrappers ---------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -99,9 +104,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
            ((uint64_t)((sbo >> 4) & 0x3fffu) << 32) | ((uint64_t)1 << 46);
 }
 
+// The descriptor of an MN-major operand without swizzle whose core matrices are
+// the same 8 rows of 16 bytes, the rows now along K: leading byte offset to the
+// next 8 K, stride byte offset to the next 8 of M or N (the other way round).
+
 // Instruction descriptor of kind::f16: FP32 accumulator (bits 4-5 = 1), BF16 A
-// and B (bits 7-9, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bits
-// 17-22, M >> 4 at bits 24-28.
+// and B (bits 7-9, 10-12 = 1), both K-major (bits 15, 16 = 0; 1: MN-major), N >> 3
+// at bits 17-22, M >> 4 at bits 24-28.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
@@ -219,7 +228,37 @@ __device__ __forceinline__ void copy_weights(uint8_t* sm, const Packed* w) {
     }
 }
 
-// cols: tensor-memory columns of the CTA (a power of 2, >= 32)
+// The same from the FP32 parameters themselves (the calls that bring their own):
+// a separate launch that packs them first took 6 us of one CTA.
+// transposed: W2 transposed too (training).
+__device__ __forceinline__ void copy_weights(uint8_t* sm, const float* __restrict__ p, bool transposed) {
+    uint16_t* w1 = reinterpret_cast<uint16_t*>(sm + SM_W1);
+    uint16_t* w2 = reinterpret_cast<uint16_t*>(sm + SM_W2);
+    uint16_t* w2t = reinterpret_cast<uint16_t*>(sm + SM_W2T);
+    float* vec = reinterpret_cast<float*>(sm + SM_VEC);
+    float* bias = reinterpret_cast<float*>(sm + SM_BIAS);
+#pragma unroll 8
+    for (int idx = threadIdx.x; idx < kH * kH; idx += kThreads) {
+        const int j = idx / kH, i = idx % kH;  // W2[j][i]: output j, input i
+        const uint16_t b = bf16_bits(p[MDAS_MLP_OFF_W2 + idx]);
+        w2[core_off(j, i, 8)] = b;
+        if (transposed) w2t[core_off(i, j, 8)] = b;
+    }
+#pragma unroll
+    for (int idx = threadIdx.x; idx < kH * kIn; idx += kThreads)
+        w1[core_off(idx / kIn, idx % kIn, 2)] = bf16_bits(p[MDAS_MLP_OFF_W1 + idx]);
+    for (int i = threadIdx.x; i < kH; i += kThreads) {
+        vec[i] = p[MDAS_MLP_OFF_B1 + i];
+        vec[kH + i] = p[MDAS_MLP_OFF_B2 + i];
+        vec[2 * kH + i] = p[MDAS_MLP_OFF_W3 + i];
+    }
+    if (threadIdx.x == 0) vec[3 * kH] = p[MDAS_MLP_OFF_B3];
+    for (int i = threadIdx.x; i < 2 * 16 * 32; i += kThreads)  // (layer, chunk, row, column)
+        bias[i] = p[((i >> 9) ? MDAS_MLP_OFF_B2 : MDAS_MLP_OFF_B1) + ((i >> 5) & 15) * 4 + (i & 3)];
+}
+
+// cols: tensor-memory columns of the CTA (a power of 2, >= 32).  The weights are
+// in shared memory when this returns if the caller copied them before.
 __device__ void ctx_open(Ctx& c, const Packed* w, unsigned* status, uint32_t cols = kTmemCols) {
     c.sm = aligned_smem();
     c.base = smem_u32(c.sm);
@@ -291,12 +330,12 @@ __device__ __forceinline__ void tmem_row(const Ctx& c, float (&acc)[kH]) {
     tmem_wait_ld();
 }
 
-// Issue `steps` MMAs over K (16 each) of A at aOff (KB K-blocks) x B at bOff
-// (after the CTA's shared-memory writes); mma_wait completes them.  biasOff >=
+// Issue `steps` MMAs over K (16 each) of A at aOff (KA K-blocks per row group) x B
+// at bOff (KB K-blocks) (after the CTA's shared-memory writes); mma_wait completes them.  biasOff >=
 // 0: the accumulators start from that bias (its 16 chunks copied into the 64
 // columns first; a chunk's descriptor has zero strides, so its one 8-row core
 // matrix stands for all 32 rows), else from zero.
-__device__ __forceinline__ void mma_issue(Ctx& c, int aOff, int bOff, int KB, int steps, int biasOff = -1) {
+__device__ __forceinline__ void mma_issue(Ctx& c, int aOff, int KA, int bOff, int KB, int steps, int biasOff = -1) {
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -304,17 +343,11 @@ __device__ __forceinline__ void mma_issue(Ctx& c, int aOff, int bOff, int KB, in
         tc_fence_after();
         if (biasOff >= 0)
             for (int j = 0; j < kH / 4; ++j) tmem_cp_32x128b_x4(c.tmem + 4 * j, smem_desc(c.base + biasOff + 128 * j, 0, 0));
-        const uint32_t sbo = (uint32_t)KB * 128u;
         for (int s = 0; s < steps; ++s)
-            mma_bf16(c.tmem, smem_desc(c.base + aOff + 256 * s, 128, sbo), smem_desc(c.base + bOff + 256 * s, 128, sbo),
-                     s > 0 || biasOff >= 0 ? 1u : 0u);
+            mma_bf16(c.tmem, smem_desc(c.base + aOff + 256 * s, 128, (uint32_t)KA * 128u),
+                     smem_desc(c.base + bOff + 256 * s, 128, (uint32_t)KB * 128u), s > 0 || biasOff >= 0 ? 1u : 0u);
         mma_commit(c.bar);
     }
-}
-
-__device__ __forceinline__ void run_mma(Ctx& c, int aOff, int bOff, int KB, int steps) {
-    mma_issue(c, aOff, bOff, KB, steps);
-    mma_wait(c);
 }
 
 // Forward of the tile whose features this thread wrote as row threadIdx.x of SM_X:
@@ -325,7 +358,7 @@ __device__ __forceinline__ void run_mma(Ctx& c, int aOff, int bOff, int KB, int 
 // memory ahead of each layer's MMAs).
 template <typename During1, typename During2>
 __device__ __forceinline__ void tile_forward(Ctx& c, float (&z2)[kH], During1 during1, During2 during2) {
-    mma_issue(c, SM_X, SM_W1, 2, 1, SM_BIAS);
+    mma_issue(c, SM_X, kHxBlocks, SM_W1, 2, 1, SM_BIAS);
     during1();
     mma_wait(c);
     float acc[kH];
@@ -333,8 +366,8 @@ __device__ __forceinline__ void tile_forward(Ctx& c, float (&z2)[kH], During1 du
 #pragma unroll
     for (int i = 0; i < kH; ++i) acc[i] = fmaxf(acc[i], 0.0f);
 #pragma unroll
-    for (int kb = 0; kb < kH / 8; ++kb) st_row8(c.sm + SM_H, threadIdx.x, kb, 8, acc + 8 * kb);
-    mma_issue(c, SM_H, SM_W2, 8, kH / 16, SM_BIAS + 16 * 128);
+    for (int kb = 0; kb < kH / 8; ++kb) st_row8(c.sm + SM_HX, threadIdx.x, kb, kHxBlocks, acc + 8 * kb);
+    mma_issue(c, SM_HX, kHxBlocks, SM_W2, 8, kH / 16, SM_BIAS + 16 * 128);
     during2();
     mma_wait(c);
     tmem_row(c, z2);
@@ -353,8 +386,8 @@ __device__ __forceinline__ float head(const Ctx& c, const float (&z2)[kH]) {
 }
 
 __device__ __forceinline__ void put_features(const Ctx& c, const float (&f)[kIn]) {
-    st_row8(c.sm + SM_X, threadIdx.x, 0, 2, f);
-    st_row8(c.sm + SM_X, threadIdx.x, 1, 2, f + 8);
+    st_row8(c.sm + SM_X, threadIdx.x, 0, kHxBlocks, f);
+    st_row8(c.sm + SM_X, threadIdx.x, 1, kHxBlocks, f + 8);
 }
 
 // ---- features --------------------------------------------------------------------
@@ -456,23 +489,20 @@ __device__ void feats_of_raw(const MdasDeviceGrid& g, const float (&raw)[MDAS_RA
 }
 
 template <int D>
-__device__ void leaf_feats(const MdasDeviceGrid& g, int leaf, int L, float (&f)[kIn], float* err) {
+__device__ void leaf_feats(const MdasDeviceGrid& g, int leaf, int L, float (&f)[kIn]) {
     float raw[MDAS_RAW_FLOATS], ne[4];
     leaf_raw<D>(g, leaf, raw);
     nbr_errors(g, leaf, L, ne);
     feats_of_raw<D>(g, raw, ne, f);
-    if (err) *err = raw[11];
-}
-
-__device__ __forceinline__ float target_of(float err) {
-    return log2f(fmaxf(err, 1e-30f)) * (1.0f / MDAS_MLP_TARGET_SCALE);
 }
 
 // ---- kernels ---------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) k_forward_rows(const Packed* __restrict__ w, const float* __restrict__ feats,
-                                                           int m, float* __restrict__ pred, unsigned* status) {
+__global__ void __launch_bounds__(kThreads) k_forward_rows(const float* __restrict__ params,
+                                                           const float* __restrict__ feats, int m,
+                                                           float* __restrict__ pred, unsigned* status) {
     Ctx c;
-    ctx_open(c, w, status);
+    copy_weights(aligned_smem(), params, false);
+    ctx_open(c, nullptr, status);
     const int tiles = (m + kRows - 1) / kRows;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int r = tile * kRows + threadIdx.x;
@@ -727,7 +757,7 @@ template <int D>
 __global__ void k_leaf_features(MdasDeviceGrid g, int L, float* __restrict__ out) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < L; r += gridDim.x * blockDim.x) {
         float f[kIn];
-        leaf_feats<D>(g, r, L, f, nullptr);
+        leaf_feats<D>(g, r, L, f);
 #pragma unroll
         for (int i = 0; i < kIn; ++i) out[(size_t)r * kIn + i] = f[i];
     }
@@ -736,36 +766,42 @@ __global__ void k_leaf_features(MdasDeviceGrid g, int L, float* __restrict__ out
 // Training: persistent CTAs over tiles of 128 rows.  Per tile: forward, then
 // dZ2 (CUDA cores), dH1 = dZ2 . W2 on the tensor cores, dZ1; the weight
 // gradients of both layers as one more tensor-core GEMM per tile,
-//   [dZ2^T ; dZ1^T] (128 x 128 rows) . [H1 | X] (128 rows x 80)
+//   [dZ2 | dZ1]^T (128 x 128 rows) . [H1 | X] (128 rows x 80)
 // whose 64 x 64 top-left block is dW2 and 64 x 16 bottom-right block is dW1
 // (the other blocks are not used), accumulated in tensor memory over all the
 // CTA's tiles; the bias-like gradients as warp reductions into shared memory.
 // At the end each CTA adds its gradient to the global one (a few thousand
 // atomics per CTA, not per tile).  BF16 operands (dZ rounded like the other
 // GEMM inputs), FP32 accumulation.
-constexpr int SM_AG = SM_Z2F;            // [dZ2^T ; dZ1^T]: 128 x 128 BF16, K-major, 16 K-blocks per row group
-constexpr int SM_BG = SM_Z1F;            // [H1 | X]^T: 80 x 128 BF16, K-major, 16 K-blocks per row group
+//
+// A tile is a chain of four waits on the tensor cores with one warp per scheduler
+// between them, so what counts is how many tiles an SM has in flight and how much
+// work lies in the chain: both row tiles are MN-major operands of the weight
+// GEMM (they used to be transposed by 208 two-byte stores per thread and took
+// 53 KB more), which leaves room for two CTAs per SM; two of the three warp
+// reductions run under the dH1 GEMM; the weight GEMM is waited for only where the
+// next tile overwrites its operands.  The gradient leaves as 16-byte additions:
+// 5313 scalar ones per CTA took as long as everything else (65,536 rows: 56 us
+// with them, 28 us with vectors).
 constexpr int kGradN = kH + kIn;         // 80 columns of the weight-gradient accumulator
 constexpr uint32_t kGradCol = 128;       // its first tensor-memory column
 constexpr uint32_t kTrainCols = 256;     // tensor-memory columns of a training CTA
-constexpr uint32_t kGradIdesc = idesc_bf16(kRows, kGradN);
-static_assert(kRows * kRows * 2 <= SM_D - SM_Z2F, "the A tile of the weight gradients fits");
-static_assert(kGradN * kRows * 2 <= SM_G - SM_Z1F, "the B tile of the weight gradients fits");
+constexpr uint32_t kGradIdesc = idesc_bf16(kRows, kGradN) | (1u << 15) | (1u << 16);  // both operands MN-major
 static_assert(kGradCol + kGradN <= kTrainCols, "tensor-memory columns");
+static_assert(MDAS_MLP_OFF_W2 % 4 == 0 && MDAS_MLP_OFF_W1 % 4 == 0, "16-byte rows of the gradient");
+static_assert(2 * (kTrainSmem + 1024) <= 227 * 1024, "two CTAs per SM");
 
-template <int D>
-__global__ void __launch_bounds__(kThreads) k_gradients(const Packed* __restrict__ w, const float* __restrict__ feats,
-                                                        const float* __restrict__ targets, MdasDeviceGrid g, int L,
-                                                        int offset, int stride, int m, float* __restrict__ grads,
-                                                        float* __restrict__ lossSum, unsigned* status) {
+__global__ void __launch_bounds__(kThreads, 2) k_gradients(const float* __restrict__ params,
+                                                           const float* __restrict__ feats,
+                                                           const float* __restrict__ targets, int m,
+                                                           float* __restrict__ grads, float* __restrict__ lossSum,
+                                                           unsigned* status) {
     Ctx c;
-    ctx_open(c, w, status, kTrainCols);
-    float* sg = reinterpret_cast<float*>(c.sm + SM_G);
-    for (int i = threadIdx.x; i < MDAS_MLP_PARAMS; i += kThreads) sg[i] = 0.0f;
-    const float* vec = reinterpret_cast<const float*>(c.sm + SM_VEC);
-    const float* w3 = vec + 2 * kH;
-    uint8_t* ag = c.sm + SM_AG;
-    uint8_t* bg = c.sm + SM_BG;
+    copy_weights(aligned_smem(), params, true);
+    ctx_open(c, nullptr, status, kTrainCols);
+    float* sg = reinterpret_cast<float*>(c.sm + SM_VG);
+    for (int i = threadIdx.x; i < 3 * kH + 1; i += kThreads) sg[i] = 0.0f;
+    const float* w3 = reinterpret_cast<const float*>(c.sm + SM_VEC) + 2 * kH;
     float* red = reinterpret_cast<float*>(c.sm + SM_RED);
     const int t = threadIdx.x;
     const int warp = t >> 5;
@@ -777,70 +813,54 @@ __global__ void __launch_bounds__(kThreads) k_gradients(const Packed* __restrict
         const bool valid = r < m;
         float f[kIn];
         float y = 0.0f;
-        if (!valid) {
 #pragma unroll
-            for (int i = 0; i < kIn; ++i) f[i] = 0.0f;
-        } else if (feats) {
-#pragma unroll
-            for (int i = 0; i < kIn; ++i) f[i] = feats[(size_t)r * kIn + i];
-            y = targets[r];
-        } else {
-            const int leaf = (int)(((long long)offset + (long long)r * stride) % L);
-            float err;
-            leaf_feats<D>(g, leaf, L, f, &err);
-            y = target_of(err);
-        }
+        for (int i = 0; i < kIn; ++i) f[i] = valid ? feats[(size_t)r * kIn + i] : 0.0f;
+        if (valid) y = targets[r];
+        if (!first) mma_wait(c);  // the last tile's weight GEMM has read [H1 | X]
         put_features(c, f);
         float z2[kH];
         tile_forward(c, z2);
         const float e = valid ? head(c, z2) - y : 0.0f;
         const float dpred = 2.0f * e / (float)m;  // 0 on rows past m
+        lossPart += e * e;
         float dz[kH];
-        {
-            float v[kH];
 #pragma unroll
-            for (int j = 0; j < kH; ++j) {
-                v[j] = dpred * fmaxf(z2[j], 0.0f);
-                dz[j] = z2[j] > 0.0f ? dpred * w3[j] : 0.0f;
-            }
-            warp_sum64(v, red + (0 * 4 + warp) * kH);  // dw3
+        for (int j = 0; j < kH; ++j) dz[j] = z2[j] > 0.0f ? dpred * w3[j] : 0.0f;
 #pragma unroll
-            for (int j = 0; j < kH; ++j) v[j] = dz[j];
-            warp_sum64(v, red + (1 * 4 + warp) * kH);  // db2
-            float d3 = dpred;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) d3 += __shfl_xor_sync(0xffffffffu, d3, o);
-            __syncthreads();  // sg zeroed (first tile); red written
-            if ((t & 31) == 0) atomicAdd(&sg[MDAS_MLP_OFF_B3], d3);
-        }
-#pragma unroll
-        for (int kb = 0; kb < kH / 8; ++kb) st_row8(c.sm + SM_D, t, kb, 8, dz + 8 * kb);
+        for (int kb = 0; kb < kH / 8; ++kb) st_row8(c.sm + SM_G, t, kb, kGBlocks, dz + 8 * kb);
         // dH1 = dZ2 . W2 on the tensor cores (B = W2 transposed, K-major)
-        run_mma(c, SM_D, SM_W2T, 8, kH / 16);
+        mma_issue(c, SM_G, kGBlocks, SM_W2T, 8, kH / 16);
+        warp_sum64(dz, red + (1 * 4 + warp) * kH);  // db2
+#pragma unroll
+        for (int j = 0; j < kH; ++j) z2[j] = dpred * fmaxf(z2[j], 0.0f);
+        warp_sum64(z2, red + (0 * 4 + warp) * kH);  // dw3
+        float d3 = dpred;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) d3 += __shfl_xor_sync(0xffffffffu, d3, o);
+        mma_wait(c);
         float dh[kH];
         tmem_row(c, dh);
-        float h1[kH];
 #pragma unroll
-        for (int kb = 0; kb < kH / 8; ++kb) ld_row8(c.sm + SM_H, t, kb, 8, h1 + 8 * kb);
+        for (int kb = 0; kb < kH / 8; ++kb) {
+            float h1[8];
+            ld_row8(c.sm + SM_HX, t, kb, kHxBlocks, h1);
 #pragma unroll
-        for (int i = 0; i < kH; ++i) dh[i] = h1[i] > 0.0f ? dh[i] : 0.0f;  // dZ1 (0 on rows past m)
-        // the operands of the weight-gradient GEMM, this thread's row r as column r
-        // (K) of [dZ2^T ; dZ1^T] and of [H1 | X]^T (the previous tile's GEMM has
-        // completed: its wait came before this tile's dH1 GEMM)
-        uint16_t* a16 = reinterpret_cast<uint16_t*>(ag);
-        uint16_t* b16 = reinterpret_cast<uint16_t*>(bg);
-#pragma unroll
-        for (int j = 0; j < kH; ++j) {
-            a16[core_off(j, t, kRows / 8)] = bf16_bits(dz[j]);
-            a16[core_off(kH + j, t, kRows / 8)] = bf16_bits(dh[j]);
-            b16[core_off(j, t, kRows / 8)] = bf16_bits(h1[j]);
+            for (int i = 0; i < 8; ++i) dh[8 * kb + i] = h1[i] > 0.0f ? dh[8 * kb + i] : 0.0f;  // dZ1 (0 on rows past m)
+            st_row8(c.sm + SM_G, t, kH / 8 + kb, kGBlocks, dh + 8 * kb);
         }
-#pragma unroll
-        for (int k = 0; k < kIn; ++k) b16[core_off(kH + k, t, kRows / 8)] = bf16_bits(f[k]);
         warp_sum64(dh, red + (2 * 4 + warp) * kH);  // db1
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
+        if (t == 0) {
+            tc_fence_after();
+            // 16 rows (K) per MMA: two 8-row groups of each tile
+            for (int ks = 0; ks < kRows / 16; ++ks)
+                mma_bf16_id(c.tmem + kGradCol, smem_desc(c.base + SM_G + 2 * ks * kGBlocks * 128, kGBlocks * 128, 128),
+                            smem_desc(c.base + SM_HX + 2 * ks * kHxBlocks * 128, kHxBlocks * 128, 128), kGradIdesc,
+                            (first && ks == 0) ? 0u : 1u);
+            mma_commit(c.bar);
+        }
         if (t < kH) {
             float a = 0.0f, b2 = 0.0f, d1 = 0.0f;
 #pragma unroll
@@ -849,50 +869,47 @@ __global__ void __launch_bounds__(kThreads) k_gradients(const Packed* __restrict
                 b2 += red[(1 * 4 + q) * kH + t];
                 d1 += red[(2 * 4 + q) * kH + t];
             }
-            sg[MDAS_MLP_OFF_W3 + t] += a;
-            sg[MDAS_MLP_OFF_B2 + t] += b2;
-            sg[MDAS_MLP_OFF_B1 + t] += d1;
+            sg[t] += a;
+            sg[kH + t] += b2;
+            sg[2 * kH + t] += d1;
         }
-        if (t == 0) {
-            tc_fence_after();
-            const uint32_t sbo = (uint32_t)(kRows / 8) * 128u;
-            for (int ks = 0; ks < kRows / 16; ++ks)
-                mma_bf16_id(c.tmem + kGradCol, smem_desc(c.base + SM_AG + 256 * ks, 128, sbo),
-                            smem_desc(c.base + SM_BG + 256 * ks, 128, sbo), kGradIdesc,
-                            (first && ks == 0) ? 0u : 1u);
-            mma_commit(c.bar);
-        }
-        mma_wait(c);
-        lossPart += e * e;
+        if ((t & 31) == 0) atomicAdd(&sg[3 * kH], d3);
         first = false;
     }
+    if (!first) mma_wait(c);  // the last weight GEMM
     // this CTA's sums into the global gradient
     float l = lossPart;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
     if ((t & 31) == 0 && l != 0.0f) atomicAdd(lossSum, l);
     if (!first) {
-        // the weight gradients: lane t of the accumulator is row t of [dZ2^T ; dZ1^T] . [H1 | X]
+        // the weight gradients: lane t of the accumulator is row t of [dZ2 | dZ1]^T . [H1 | X]
         float acc[kGradN];
         const uint32_t lane = (threadIdx.x & ~31u) << 16;
 #pragma unroll
         for (int q = 0; q < kGradN / 16; ++q) tmem_ld16(c.tmem + lane + kGradCol + 16 * q, acc + 16 * q);
         tmem_wait_ld();
-        if (t < kH) {
+        // rows 0-63: 64 columns of dW2, rows 64-127: 16 of dW1, each row contiguous
+        float* out = grads + (t < kH ? MDAS_MLP_OFF_W2 + t * kH : MDAS_MLP_OFF_W1 + (t - kH) * kIn);
+        if ((reinterpret_cast<uintptr_t>(grads) & 15) == 0) {
 #pragma unroll
-            for (int i = 0; i < kH; ++i)
-                if (acc[i] != 0.0f) atomicAdd(&grads[MDAS_MLP_OFF_W2 + t * kH + i], acc[i]);
+            for (int i = 0; i < kGradN; i += 4)
+                if (t < kH ? i < kH : i >= kH)
+                    atomicAdd(reinterpret_cast<float4*>(out + (i < kH ? i : i - kH)),
+                              make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]));
         } else {
 #pragma unroll
-            for (int k = 0; k < kIn; ++k)
-                if (acc[kH + k] != 0.0f) atomicAdd(&grads[MDAS_MLP_OFF_W1 + (t - kH) * kIn + k], acc[kH + k]);
+            for (int i = 0; i < kGradN; ++i)
+                if (t < kH ? i < kH : i >= kH) atomicAdd(out + (i < kH ? i : i - kH), acc[i]);
         }
     }
     __syncthreads();
-    for (int i = t; i < MDAS_MLP_PARAMS; i += kThreads) {
-        const float v = sg[i];
-        if (v != 0.0f) atomicAdd(&grads[i], v);
+    if (t < kH) {
+        if (sg[t] != 0.0f) atomicAdd(&grads[MDAS_MLP_OFF_W3 + t], sg[t]);
+        if (sg[kH + t] != 0.0f) atomicAdd(&grads[MDAS_MLP_OFF_B2 + t], sg[kH + t]);
+        if (sg[2 * kH + t] != 0.0f) atomicAdd(&grads[MDAS_MLP_OFF_B1 + t], sg[2 * kH + t]);
     }
+    if (t == 0 && sg[3 * kH] != 0.0f) atomicAdd(&grads[MDAS_MLP_OFF_B3], sg[3 * kH]);
     ctx_close(c);
 }
 
@@ -960,13 +977,13 @@ cudaError_t set_test_wait_limit(int polls) {
     return cudaMemcpyToSymbol(test_wait_limit, &v, sizeof(int));
 }
 
-cudaError_t forward(const Packed* w, const float* features, int m, float* pred, unsigned* status, cudaStream_t s) {
+cudaError_t forward(const float* params, const float* features, int m, float* pred, unsigned* status, cudaStream_t s) {
     if (m <= 0) return cudaSuccess;
     cudaError_t e = set_smem(k_forward_rows, kFwdSmem);
     if (e != cudaSuccess) return e;
     const int tiles = (m + kRows - 1) / kRows;
     const int grid = tiles < sm_count() * 4 ? tiles : sm_count() * 4;
-    k_forward_rows<<<grid, kThreads, kFwdSmem, s>>>(w, features, m, pred, status);
+    k_forward_rows<<<grid, kThreads, kFwdSmem, s>>>(params, features, m, pred, status);
     return cudaGetLastError();
 }
 
@@ -1003,28 +1020,20 @@ cudaError_t leaf_features(const MdasDeviceGrid& g, int L, float* features, cudaS
     return cudaGetLastError();
 }
 
-cudaError_t gradients(const Packed* w, const float* features, const float* targets, const MdasDeviceGrid* g, int L,
-                      int offset, int stride, int m, float* grads, float* lossSum, unsigned* status, cudaStream_t s) {
+cudaError_t gradients(const float* params, const float* features, const float* targets, int m, float* grads,
+                      float* lossSum, unsigned* status, cudaStream_t s) {
     if (m <= 0) return cudaSuccess;
-    if (!features && (!g || L <= 0)) return cudaErrorInvalidValue;
     const int tiles = (m + kRows - 1) / kRows;
-    MdasDeviceGrid none{};
-    none.D = 4;
-    const MdasDeviceGrid& gg = g ? *g : none;
-    cudaError_t e = cudaSuccess;
-    const int grid = tiles < sm_count() ? tiles : sm_count();  // persistent: one CTA per SM (shared memory)
-    MLP_SWITCH_D(gg.D, (e = set_smem(k_gradients<DD>, kTrainSmem),
-                        e == cudaSuccess ? (k_gradients<DD><<<grid, kThreads, kTrainSmem, s>>>(
-                                                w, features, targets, gg, L, offset, stride, m, grads, lossSum, status),
-                                            0)
-                                         : 0));
-    return e != cudaSuccess ? e : cudaGetLastError();
+    const int most = 2 * sm_count();  // persistent: two CTAs per SM
+    cudaError_t e = set_smem(k_gradients, kTrainSmem);
+    if (e != cudaSuccess) return e;
+    k_gradients<<<tiles < most ? tiles : most, kThreads, kTrainSmem, s>>>(params, features, targets, m, grads, lossSum,
+                                                                          status);
+    return cudaGetLastError();
 }
 
-cudaError_t adam(float* params, float* m1, float* m2, float* grads, int step, float lr, Packed* packed,
-                 cudaStream_t s) {
+cudaError_t adam(float* params, float* m1, float* m2, float* grads, int step, float lr, cudaStream_t s) {
     k_adam<<<(MDAS_MLP_PARAMS + 255) / 256, 256, 0, s>>>(params, m1, m2, grads, step, lr);
-    k_pack<<<1, 1024, 0, s>>>(params, packed);
     return cudaGetLastError();
 }
 

@@ -50,8 +50,9 @@ struct Packed {
 
 // FP32 parameters -> packed copy.
 cudaError_t pack(const float* params, Packed* packed, cudaStream_t s);
-// pred[i] = MLP(features[i]) for m rows of 16 features (FP32, converted to BF16).
-cudaError_t forward(const Packed* w, const float* features, int m, float* pred, unsigned* status, cudaStream_t s);
+// pred[i] = MLP(features[i]) for m rows of 16 features (FP32, converted to BF16);
+// params: FP32, MDAS_MLP_PARAMS.
+cudaError_t forward(const float* params, const float* features, int m, float* pred, unsigned* status, cudaStream_t s);
 // Priorities of the grid's leaves: log2(plain error) / 32 plus the network's
 // correction, for every leaf (mode 0), the leaves whose error the last errors
 // pass recomputed (1: features gathered; 3: from the raw rows that pass wrote
@@ -67,16 +68,12 @@ cudaError_t predict_leaves(const MdasDeviceGrid& g, int L, int mode, const Packe
 cudaError_t batch_predict(const MdasBatchImage* imgs, int n, int D, unsigned* status, cudaStream_t s);
 // Features of the grid's leaves (training data, tests).
 cudaError_t leaf_features(const MdasDeviceGrid& g, int L, float* features, cudaStream_t s);
-// Adds the gradients of the mean squared error over m rows to grads (FP32,
-// MDAS_MLP_PARAMS) and the sum of squared errors to *lossSum.  Rows come from
-// features/targets if given, else from the grid's leaves (row r = leaf
-// (offset + r * stride) % L, target = its plain log2(error) / MDAS_MLP_TARGET_SCALE).
-cudaError_t gradients(const Packed* w, const float* features, const float* targets, const MdasDeviceGrid* g, int L,
-                      int offset, int stride, int m, float* grads, float* lossSum, unsigned* status, cudaStream_t s);
-// One Adam step (bias-corrected, step >= 1) on params with grads (zeroed
-// afterwards), then repacks.
-cudaError_t adam(float* params, float* m1, float* m2, float* grads, int step, float lr, Packed* packed,
-                 cudaStream_t s);
+// Adds the gradients of the mean squared error over m rows of features and
+// targets to grads (FP32, MDAS_MLP_PARAMS) and the sum of squared errors to *lossSum.
+cudaError_t gradients(const float* params, const float* features, const float* targets, int m, float* grads,
+                      float* lossSum, unsigned* status, cudaStream_t s);
+// One Adam step (bias-corrected, step >= 1) on params with grads (zeroed afterwards).
+cudaError_t adam(float* params, float* m1, float* m2, float* grads, int step, float lr, cudaStream_t s);
 
 // Polls after which the MMA waits report a timeout (<= 0: their own limit); a test hook.
 cudaError_t set_test_wait_limit(int polls);
