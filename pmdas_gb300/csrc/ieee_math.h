@@ -46,9 +46,67 @@ MDAS_HD float mdas_u2f(uint32_t u) {
 #endif
 }
 
+// Device code built with the reference's fast-math flags (MDAS_REFERENCE_ARITH)
+// spells the operations below out in PTX, so that nothing of them is contracted,
+// approximated or flushed there; elsewhere the compiler's flags see to it
+// (build.py).
+#if defined(__CUDA_ARCH__) && defined(MDAS_REFERENCE_ARITH)
+#define MDAS_EXPLICIT_PTX 1
+#else
+#define MDAS_EXPLICIT_PTX 0
+#endif
+
 // Fused multiply-add with a single rounding; fmaf is correctly rounded on the
 // device (fma.rn.f32) and in any conforming C library.
-MDAS_HD float mdas_fma(float a, float b, float c) { return fmaf(a, b, c); }
+MDAS_HD float mdas_fma(float a, float b, float c) {
+#if MDAS_EXPLICIT_PTX
+    float r;
+    asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+#else
+    return fmaf(a, b, c);
+#endif
+}
+
+// The other operations, correctly rounded and with subnormals kept (the integrand
+// also runs inside kernels built with the fast-math flags).
+#if MDAS_EXPLICIT_PTX
+#define MDAS_OP2(NAME, PTX, OP)                                             \
+    MDAS_HD float NAME(float a, float b) {                                  \
+        float r;                                                            \
+        asm(PTX ".rn.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));          \
+        return r;                                                           \
+    }
+#define MDAS_CMP(NAME, PTX, OP)                                             \
+    MDAS_HD bool NAME(float a, float b) {                                   \
+        int r;                                                              \
+        asm("{\n .reg .pred p;\n setp." PTX ".f32 p, %1, %2;\n selp.s32 %0, 1, 0, p;\n}" : "=r"(r) : "f"(a), "f"(b)); \
+        return r != 0;                                                      \
+    }
+#else
+#define MDAS_OP2(NAME, PTX, OP) MDAS_HD float NAME(float a, float b) { return a OP b; }
+#define MDAS_CMP(NAME, PTX, OP) MDAS_HD bool NAME(float a, float b) { return a OP b; }
+#endif
+MDAS_OP2(mdas_add, "add", +)
+MDAS_OP2(mdas_sub, "sub", -)
+MDAS_OP2(mdas_mul, "mul", *)
+MDAS_OP2(mdas_div, "div", /)
+MDAS_CMP(mdas_lt, "lt", <)
+MDAS_CMP(mdas_le, "le", <=)
+#undef MDAS_OP2
+#undef MDAS_CMP
+
+MDAS_HD float mdas_neg(float a) { return mdas_u2f(mdas_f2u(a) ^ 0x80000000u); }
+
+MDAS_HD float mdas_sqrt(float a) {
+#if MDAS_EXPLICIT_PTX
+    float r;
+    asm("sqrt.rn.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+#else
+    return sqrtf(a);
+#endif
+}
 
 // 2^n for integer n in [-149, 127], exact.
 MDAS_HD float mdas_exp2i(int n) {
@@ -119,13 +177,13 @@ MDAS_HD float mdas_powf(float x, float y) {
 
 // sin and cos of phi in [-pi/4, pi/4] (Taylor series to degree 11 / 10).
 MDAS_HD void mdas_sincos_quarter(float phi, float* s, float* c) {
-    const float t2 = phi * phi;
+    const float t2 = mdas_mul(phi, phi);
     float ps = -2.50521084e-8f;            // -1/11!
     ps = mdas_fma(ps, t2, 2.75573192e-6f); // 1/9!
     ps = mdas_fma(ps, t2, -1.98412698e-4f);// -1/7!
     ps = mdas_fma(ps, t2, 8.33333333e-3f); // 1/5!
     ps = mdas_fma(ps, t2, -0.166666667f);  // -1/3!
-    ps = ps * t2;
+    ps = mdas_mul(ps, t2);
     *s = mdas_fma(phi, ps, phi);
     float pc = -2.75573192e-7f;            // -1/10!
     pc = mdas_fma(pc, t2, 2.48015873e-5f); // 1/8!

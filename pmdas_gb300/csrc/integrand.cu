@@ -13,11 +13,12 @@
 #include "integrand.h"
 #include "grid_types.h"
 #include "scene.h"
+#include "shade.cuh"
 
 namespace {
 
 // ---- disc culling ---------------------------------------------------------------------
-__host__ __device__ inline bool mdas_culled_kind(int kind) {
+bool mdas_culled_kind(int kind) {
     return kind == MDAS_SCENE_DISCS_MB || kind == MDAS_SCENE_DISCS_DOF || kind == MDAS_SCENE_DISCS_MBDOF;
 }
 
@@ -54,88 +55,32 @@ __device__ bool cull_may_cover(const MdasScene& sc, const float* p, float x0, fl
     return !(dist > reach + 1.0e-3f * scale);
 }
 
-// One warp per (tile, mask word): lane b tests disc 32 * word + b, the
-// ballot is the word.
+// One warp per tile: its lanes test 32 discs at a time, in the order in which the
+// full scan tests them (integrand.h: motion blur from the last disc, depth of field
+// from the first), and append those kept to the tile's list (shade.cuh).
 __global__ void __launch_bounds__(256) k_build_cull(MdasScene sc, const float* __restrict__ prims,
-                                                     unsigned* __restrict__ masks) {
+                                                     unsigned* __restrict__ lists) {
     constexpr int T = MDAS_CULL_TILES;
-    const int words = (sc.count + 31) / 32;
-    const int total = T * T * words;
     const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * (blockDim.x >> 5);
-    for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < total; i += warps) {
-        const int tile = i / words, w = i - tile * words;
+    for (int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < T * T; tile += warps) {
         const int tx = tile % T, ty = tile / T;
         const float pad = 1.0e-4f;
         const float x0 = (float)tx / T - pad, x1 = (float)(tx + 1) / T + pad;
         const float y0 = (float)ty / T - pad, y1 = (float)(ty + 1) / T + pad;
-        const int k = 32 * w + lane;
-        const bool may = k < sc.count && cull_may_cover(sc, prims + MDAS_PRIM_STRIDE * k, x0, x1, y0, y1);
-        const unsigned m = __ballot_sync(0xffffffffu, may);
-        if (lane == 0) masks[i] = m;
-    }
-}
-
-__device__ __forceinline__ int cull_tile(float px, float py) {
-    constexpr int T = MDAS_CULL_TILES;
-    const int tx = min(max((int)(px * (float)T), 0), T - 1);
-    const int ty = min(max((int)(py * (float)T), 0), T - 1);
-    return ty * T + tx;
-}
-
-// mdas_shade over the tile's candidate discs: the same tests in the same order
-// as the full scans of integrand.h (the direct-light kind is not culled).
-__device__ void shade_culled(const MdasScene& sc, const float* prims, const unsigned* __restrict__ cull,
-                             const float* c, float* out) {
-    const int words = (sc.count + 31) / 32;
-    float R = sc.background, G = sc.background, B = sc.background;
-    if (sc.kind == MDAS_SCENE_DISCS_MB) {
-        const float px = c[0] / sc.scaleX;
-        const float py = c[1] / sc.scaleY;
-        const float t = c[2];
-        const unsigned* m = cull + (size_t)cull_tile(px, py) * words;
-        // the last listed covering disc wins: from the back
-        for (int w = words - 1; w >= 0; --w) {
-            unsigned bits = m[w];
-            while (bits) {
-                const int b = 31 - __clz(bits);
-                bits &= ~(1u << b);
-                const float* p = prims + MDAS_PRIM_STRIDE * (32 * w + b);
-                if (mdas_disc_mb_covers(p, px, py, t)) {
-                    R = p[8];
-                    G = p[9];
-                    B = p[10];
-                    goto done;
-                }
-            }
+        unsigned* list = lists + (size_t)tile * mdas_cull_stride(sc.count);
+        unsigned short* entries = reinterpret_cast<unsigned short*>(list + 1);
+        int n = 0;
+        for (int base = 0; base < sc.count; base += 32) {
+            const int i = base + lane;
+            const int k = sc.kind == MDAS_SCENE_DISCS_MB ? sc.count - 1 - i : i;
+            const bool may = i < sc.count && cull_may_cover(sc, prims + MDAS_PRIM_STRIDE * k, x0, x1, y0, y1);
+            const unsigned m = __ballot_sync(0xffffffffu, may);
+            if (may) entries[n + __popc(m & ((1u << lane) - 1u))] = (unsigned short)k;
+            n += __popc(m);
         }
-    } else if (sc.kind == MDAS_SCENE_DISCS_DOF || sc.kind == MDAS_SCENE_DISCS_MBDOF) {
-        const int moving = sc.kind == MDAS_SCENE_DISCS_MBDOF;
-        float t, lx, ly, wx, wy;
-        mdas_dof_ray(&sc, c, moving, &t, &lx, &ly, &wx, &wy);
-        const unsigned* m = cull + (size_t)cull_tile(c[0] / sc.scaleX, c[1] / sc.scaleY) * words;
-        for (int w = 0; w < words; ++w) {
-            unsigned bits = m[w];
-            while (bits) {
-                const int b = __ffs(bits) - 1;
-                bits &= bits - 1u;
-                const float* p = prims + MDAS_PRIM_STRIDE * (32 * w + b);
-                if (mdas_disc_dof_covers(p, lx, ly, wx, wy, t, moving)) {
-                    R = p[8];
-                    G = p[9];
-                    B = p[10];
-                    goto done;
-                }
-            }
-        }
-    } else {
-        mdas_shade(&sc, prims, c, out);
-        return;
+        if (lane == 0) list[0] = (unsigned)n;
     }
-done:
-    out[0] = R;
-    out[1] = G;
-    out[2] = B;
 }
 
 template <int D>
@@ -270,7 +215,7 @@ __device__ __forceinline__ double lanes_sum(double v) {
 // uniform, radiance accumulated in FP64.  T lanes share a pixel's stream and
 // its samples (the lanes of a warp then test the same few discs), so that a
 // 256 x 256 image fills the GPU too.
-// cull (may be null): the scene's culling masks; the samples' values are the full
+// cull (may be null): the scene's culling lists; the samples' values are the full
 // scan's either way.
 // 4-D depth of field, 256 discs, 256 x 256 at 1024 spp: 0.89 ms; 12.8 ms with one
 // thread per pixel testing every disc from the front.
@@ -453,15 +398,14 @@ cudaError_t mdas_launch_leaf_true_errors(const MdasScene& sc, const float* d_pri
 
 size_t mdas_cull_words(const MdasScene& sc) {
     if (!mdas_culled_kind(sc.kind) || sc.count <= 0) return 0;
-    return (size_t)MDAS_CULL_TILES * MDAS_CULL_TILES * (size_t)((sc.count + 31) / 32);
+    return (size_t)MDAS_CULL_TILES * MDAS_CULL_TILES * (size_t)mdas_cull_stride(sc.count);
 }
 
-cudaError_t mdas_launch_build_cull(const MdasScene& sc, const float* d_prims, unsigned* masks, cudaStream_t s) {
-    const size_t words = mdas_cull_words(sc);
-    if (words == 0) return cudaSuccess;
-    if (!masks) return cudaErrorInvalidValue;
-    const size_t blocks = (words + 7) / 8;  // 8 warps per block, one mask word per warp
-    k_build_cull<<<(unsigned)(blocks < 8192 ? blocks : 8192), 256, 0, s>>>(sc, d_prims, masks);
+cudaError_t mdas_launch_build_cull(const MdasScene& sc, const float* d_prims, unsigned* lists, cudaStream_t s) {
+    if (mdas_cull_words(sc) == 0) return cudaSuccess;
+    if (!lists) return cudaErrorInvalidValue;
+    // (8 warps per block, one tile per warp)
+    k_build_cull<<<MDAS_CULL_TILES * MDAS_CULL_TILES / 8, 256, 0, s>>>(sc, d_prims, lists);
     return cudaGetLastError();
 }
 
