@@ -75,7 +75,7 @@ __device__ __forceinline__ int2 batch_run(int total) {
 }
 
 // A CTA's maximum and sum added to two words (block-uniform call of 256 threads;
-// s_red: 16 words of shared memory).
+// s_red: 16 words of shared memory; sumOut may be null).
 __device__ __forceinline__ void block_flush(unsigned m, unsigned c, unsigned* s_red, unsigned* maxOut, unsigned* sumOut) {
     m = __reduce_max_sync(0xffffffffu, m);
     c = __reduce_add_sync(0xffffffffu, c);
@@ -90,7 +90,7 @@ __device__ __forceinline__ void block_flush(unsigned m, unsigned c, unsigned* s_
         c = __reduce_add_sync(0xffffffffu, threadIdx.x < 8 ? s_red[8 + threadIdx.x] : 0u);
         if (threadIdx.x == 0) {
             if (m) atomicMax(maxOut, m);
-            if (c) atomicAdd(sumOut, c);
+            if (sumOut && c) atomicAdd(sumOut, c);
         }
     }
 }
@@ -248,66 +248,82 @@ __global__ void k_batch_verdict(const MdasBatchImage* __restrict__ imgs, int n) 
     st->keptMax = 0u;  // taken by this pass's predMax; the adaptive pass sets it anew
 }
 
-// ---- errors: full on an image's first pass, its split children after
+// ---- errors of every active image's initial leaves (those of later split children
+// come with the new samples' values).
 // A thread keeps its running maximum and count while the CTA's chunks stay in
 // one image; the CTA adds them to that image's counters when it moves on.
 template <int D>
-__global__ void __launch_bounds__(256, 5) k_batch_errors(const MdasBatchImage* __restrict__ imgs, int n) {
+__global__ void __launch_bounds__(256) k_batch_initial_errors(const MdasBatchImage* __restrict__ imgs, int n) {
     __shared__ int s_pre[MDAS_MAX_BATCH + 1];
     __shared__ unsigned s_warp[8], s_red[16];
     const int total = batch_prefix(n, s_pre, s_warp, [&](int i) {
         const MdasCounts* c = imgs[i].g.counts;
-        if (!c->active) return 0;
-        const int items = c->passes == 0 ? c->L : 2 * c->newL;
-        return ceil_div(items, 256) > 0 ? ceil_div(items, 256) : 1;  // one chunk carries gerrNext
+        return c->active ? ceil_div(c->L, 256) : 0;
     });
     int cur = -1;  // the image the running values belong to (uniform across the block)
     float maxError = 0.0f;
-    unsigned recomputed = 0;
+    unsigned computed = 0;
     auto flush = [&]() {
         MdasCounts* c = imgs[cur].g.counts;
-        block_flush(__float_as_uint(maxError), recomputed, s_red, &c->gerr, reinterpret_cast<unsigned*>(&c->recomputed));
+        block_flush(__float_as_uint(maxError), computed, s_red, &c->gerr, reinterpret_cast<unsigned*>(&c->recomputed));
+        maxError = 0.0f;
+        computed = 0;
     };
     const int2 run = batch_run(total);
     for (int ch = run.x; ch < run.y; ++ch) {
         const int i = batch_image_of(s_pre, n, ch);
         const MdasDeviceGrid& g = imgs[i].g;
-        const MdasCounts* cnt = g.counts;
-        const bool dirty = cnt->passes > 0;
-        const int newL = cnt->newL;
-        const int items = dirty ? 2 * newL : cnt->L;
-        const int firstRight = cnt->L - newL;
-        const int k = (ch - s_pre[i]) * 256 + threadIdx.x;
         if (i != cur) {
             if (cur >= 0) flush();
             cur = i;
-            maxError = dirty ? __uint_as_float(cnt->gerrCarry) : 0.0f;
-            recomputed = 0;
         }
-        if (k < items && dirty) {
-            // split children from the splitting pass's lists (no leaf record read);
-            // learned images also complete the child's raw feature row.  The two
-            // children of a split in neighbouring lanes (item kk: left children
-            // first, then right ones, as the lists and rows are laid out)
-            const int kk = (k & 1) ? newL + (k >> 1) : (k >> 1);
-            const bool left = kk < newL;
-            const int4 sp = left ? g.splitL[kk] : g.splitR[kk - newL];
-            const int nodeIndex = left ? sp.z : firstRight + (kk - newL);
-            MdasLumStats lum;
-            const float error = node_error<D>(g, make_int4(sp.x, sp.y, left ? ~D : sp.z, ~D), __int_as_float(sp.w),
-                                              g.featRaw ? &lum : nullptr);
-            if (g.featRaw) mdas_raw_store_stats(g.featRaw + (size_t)kk * MDAS_RAW_FLOATS, lum, error);
-            g.errors[nodeIndex] = error;
-            recomputed++;
+        const int k = (ch - s_pre[i]) * 256 + threadIdx.x;
+        if (k < g.counts->L) {
+            const float error = leaf_error<D>(g, k);
+            g.errors[k] = error;
+            ++computed;
             maxError = fmaxf(maxError, error);
-        } else if (k < items) {
-            float error = g.errors[k];
-            if (error < 0.0f) {
-                error = leaf_error<D>(g, k);
-                g.errors[k] = error;
-                recomputed++;
-            }
-            maxError = fmaxf(maxError, error);
+        }
+    }
+    if (cur >= 0) flush();
+}
+
+// ---- the pass's new samples: values, and errors of the split children
+// (k_render_values over the images)
+template <int D>
+__global__ void __launch_bounds__(256, 4) k_batch_values(const MdasBatchImage* __restrict__ imgs,
+                                                      const MdasBatchScene* __restrict__ scenes, int n) {
+    __shared__ int s_pre[MDAS_MAX_BATCH + 1];
+    __shared__ unsigned s_warp[8], s_red[16];
+    pdl_wait();
+    // (an image without an accepted leaf gets a chunk too: one CTA sets its g_error)
+    const int total = batch_prefix(n, s_pre, s_warp, [&](int i) {
+        const MdasDeviceGrid& g = imgs[i].g;
+        return g.counts->active ? max(ceil_div(g.counts->newN, 256), 1) : 0;
+    });
+    int cur = -1;  // the image of the running maximum (uniform across the block)
+    float maxError = 0.0f;
+    auto flush = [&]() {
+        MdasCounts* c = imgs[cur].g.counts;
+        block_flush(__float_as_uint(maxError), 0u, s_red, &c->gerr, nullptr);
+        maxError = 0.0f;
+    };
+    const int2 run = batch_run(total);
+    for (int ch = run.x; ch < run.y; ++ch) {
+        const int i = batch_image_of(s_pre, n, ch);
+        const MdasDeviceGrid& g = imgs[i].g;
+        if (i != cur) {
+            if (cur >= 0) flush();
+            cur = i;
+        }
+        const bool more = g.ctl->more != 0;
+        const MdasBatchScene& b = scenes[i];
+        const float m = render_sample<D>(g, b.sc, b.prims, b.cull, (ch - s_pre[i]) * 256 + threadIdx.x, g.counts->newN,
+                                         g.ctl->N0, g.ctl->L0, more);
+        maxError = fmaxf(maxError, m);
+        if (more && ch == s_pre[i] && threadIdx.x == 0) {  // the image's first chunk
+            maxError = fmaxf(maxError, __uint_as_float(g.counts->gerrCarry));
+            g.counts->recomputed = 2 * g.counts->newL;
         }
     }
     if (cur >= 0) flush();
@@ -357,14 +373,14 @@ __global__ void __launch_bounds__(256, LEARNED ? 3 : 4) k_batch_decide(const Mda
 }
 
 // ---- adaptive pass: scan (one CTA of 1024 threads per image)
-__global__ void __launch_bounds__(1024) k_batch_scan(const MdasBatchImage* __restrict__ imgs, int n) {
+__global__ void __launch_bounds__(1024) k_batch_scan(const MdasBatchImage* __restrict__ imgs, int n, int maxPasses) {
     pdl_wait();
     pdl_launch_dependents();
     __shared__ unsigned s_sel[32], s_split[32];
     if ((int)blockIdx.x >= n) return;
     const MdasDeviceGrid& g = imgs[blockIdx.x].g;
     if (!g.counts->active) return;
-    scan_image(g, s_sel, s_split);
+    scan_image(g, s_sel, s_split, imgs[blockIdx.x].budget, maxPasses);
 }
 
 // ---- adaptive pass: place (one thread per accepted leaf), staged and
@@ -421,7 +437,7 @@ __global__ void __launch_bounds__(256, D >= 5 ? 2 : 3) k_batch_place(const MdasB
         if (cur.count > 0) {
             const MdasDeviceGrid& g = imgs[cur.img].g;
             place_warp<D>(g, cur.tile, cur.pre, cur.e, g.ctl->N0, g.ctl->L0, cur.kb, cur.count, s_rec[buf][warp],
-                          s_new[D == 4 ? 0 : warp]);
+                          s_new[D == 4 ? 0 : warp], true);
         }
         __syncwarp();  // the buffer is refilled two iterations on
         if (!more) break;
@@ -505,9 +521,16 @@ cudaError_t batch_set_counts(const MdasBatchImage* imgs, int n, cudaStream_t s) 
     return cudaGetLastError();
 }
 
-cudaError_t batch_errors(const MdasBatchImage* imgs, int n, int D, int grid, cudaStream_t s) {
-    MDAS_BATCH_SWITCH_D(D, (k_batch_errors<DD><<<grid, 256, 0, s>>>(imgs, n)));
+cudaError_t batch_initial_errors(const MdasBatchImage* imgs, int n, int D, int grid, cudaStream_t s) {
+    MDAS_BATCH_SWITCH_D(D, (k_batch_initial_errors<DD><<<grid, 256, 0, s>>>(imgs, n)));
     return cudaGetLastError();
+}
+
+cudaError_t batch_values(const MdasBatchImage* imgs, const MdasBatchScene* scenes, int n, int D, int grid,
+                         cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    MDAS_BATCH_SWITCH_D(D, (e = launch_pdl(k_batch_values<DD>, grid, 256, s, imgs, scenes, n)));
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t batch_reset(const MdasBatchImage* imgs, int n, int which, cudaStream_t s) {
@@ -536,8 +559,8 @@ cudaError_t batch_decide(const MdasBatchImage* imgs, int n, int D, int K, bool l
     return cudaGetLastError();
 }
 
-cudaError_t batch_scan(const MdasBatchImage* imgs, int n, cudaStream_t s) {
-    cudaError_t e = launch_pdl(k_batch_scan, n, 1024, s, imgs, n);
+cudaError_t batch_scan(const MdasBatchImage* imgs, int n, int maxPasses, cudaStream_t s) {
+    cudaError_t e = launch_pdl(k_batch_scan, n, 1024, s, imgs, n, maxPasses);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }

@@ -62,7 +62,7 @@ struct mdas_grid {
     cudaStream_t stream = nullptr;
     int device = 0;
     int numSMs = 1;
-    int occ[MDAS_K_COUNT] = {1, 1, 1, 1, 1};
+    int occ[MDAS_K_COUNT] = {1, 1, 1, 1, 1, 1};
     int N = 0, L = 0, newN = 0, newL = 0;
     bool initialized = false;
     // errorsClean: every leaf error is >= 0 (an errors pass ran since the last change).
@@ -900,20 +900,14 @@ namespace {
 
 constexpr int kMaxGraphPasses = 1 << 20;  // safety stop of the device-side loop
 
-cudaError_t launch_errors_auto(mdas_grid* g, int grid, cudaStream_t s) {
-    return g->arith == MDAS_ARITH_IEEE ? mdas_ieee::compute_errors_auto(g->dg, grid, s)
-                                       : mdas_fast::compute_errors_auto(g->dg, grid, s);
-}
+#define MDAS_GRID_CALL(g, FN, ...) \
+    ((g)->arith == MDAS_ARITH_IEEE ? mdas_ieee::FN(__VA_ARGS__) : mdas_fast::FN(__VA_ARGS__))
 
-cudaError_t launch_adaptive_on(mdas_grid* g, int gridDecide, int gridPlace, cudaStream_t s) {
-    return g->arith == MDAS_ARITH_IEEE ? mdas_ieee::adaptive_sampling(g->dg, gridDecide, gridPlace, s)
-                                       : mdas_fast::adaptive_sampling(g->dg, gridDecide, gridPlace, s);
-}
-
-// Builds the whole render as one graph: initial sampling, integrand, a
-// conditional while node around {errors, adaptive pass, integrand for the new
-// samples, loop condition}, integrate.  Every kernel has a fixed persistent
-// grid and reads the leaf and sample counts from device memory.
+// Builds the whole render as one graph: initial sampling, integrand, errors of the
+// initial leaves, a conditional while node around {decide, scan with the loop's
+// condition, place, values of the new samples with the errors of the split
+// children}, integrate.  Every kernel has a fixed persistent grid and reads the
+// leaf and sample counts from device memory.
 cudaError_t learned_queue(mdas_grid* g, int L, cudaStream_t s);
 
 int build_render_graph(mdas_grid* g, mdas_scene* s, int budget, float* pixels, int width, int height) {
@@ -934,6 +928,7 @@ int build_render_graph(mdas_grid* g, mdas_scene* s, int budget, float* pixels, i
     const int gDecide = g->numSMs * (g->occ[MDAS_K_DECIDE] > 0 ? g->occ[MDAS_K_DECIDE] : 1);
     const int gPlace = g->numSMs * (g->occ[MDAS_K_ADAPTIVE] > 0 ? g->occ[MDAS_K_ADAPTIVE] : 1);
     const int gInt = g->numSMs * (g->occ[MDAS_K_INTEGRATE] > 0 ? g->occ[MDAS_K_INTEGRATE] : 1);
+    const int gVal = g->numSMs * (g->occ[MDAS_K_RENDER_VALUES] > 0 ? g->occ[MDAS_K_RENDER_VALUES] : 1);
     const int gEval = g->numSMs * 16;  // integrand CTAs (16 per SM measured 1 % faster per render than 8)
     cudaStream_t cs = g->captureStream, bs = g->bodyStream;
     cudaGraph_t graph = nullptr;
@@ -952,6 +947,8 @@ int build_render_graph(mdas_grid* g, mdas_scene* s, int budget, float* pixels, i
     if (e != cudaSuccess) return fail(e);
     k_set_counts<<<1, 1, 0, cs>>>(d.counts, (int)N0, (int)L0);
     e = mdas_launch_evaluate(s->desc, s->d_prims, s->d_cull, d.coords, d.values, d.D, nullptr, 0, (int)N0, gEval, cs);
+    // (a render without a pass leaves the errors uncomputed, as the host loop does)
+    if (e == cudaSuccess && firstPass) e = MDAS_GRID_CALL(g, compute_errors, d, gErr, false, cs);
     if (e != cudaSuccess) return fail(e);
     // the conditional while node
     cudaStreamCaptureStatus status;
@@ -977,18 +974,15 @@ int build_render_graph(mdas_grid* g, mdas_scene* s, int budget, float* pixels, i
     // loop body, captured into the conditional node's child graph
     e = cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
     if (e != cudaSuccess) return fail(e);
-    cudaError_t eb = launch_errors_auto(g, gErr, bs);
-    if (eb == cudaSuccess && g->learned) {
+    cudaError_t eb = cudaSuccess;
+    if (g->learned) {
         eb = learned_queue(g, -1, bs);  // predictions and the judge's verdict for this pass
         g->dg.priority = g->lPred;
     }
-    if (eb == cudaSuccess) eb = launch_adaptive_on(g, gDecide, gPlace, bs);
+    if (eb == cudaSuccess)
+        eb = MDAS_GRID_CALL(g, render_pass, d, s->desc, s->d_prims, s->d_cull, handle, budget, kMaxGraphPasses, gDecide,
+                            gPlace, gVal, bs);
     g->dg.priority = nullptr;
-    if (eb == cudaSuccess)
-        eb = mdas_launch_evaluate(s->desc, s->d_prims, s->d_cull, d.coords, d.values, d.D, d.counts, 0, 0, gEval, bs);
-    if (eb == cudaSuccess)
-        eb = g->arith == MDAS_ARITH_IEEE ? mdas_ieee::loop_condition(d, handle, budget, kMaxGraphPasses, bs)
-                                         : mdas_fast::loop_condition(d, handle, budget, kMaxGraphPasses, bs);
     cudaGraph_t bodyOut = nullptr;
     e = cudaStreamEndCapture(bs, &bodyOut);
     if (eb != cudaSuccess || e != cudaSuccess) return fail(eb != cudaSuccess ? eb : e);
@@ -1107,13 +1101,15 @@ cudaError_t enqueue_batch_prologue(mdas_batch* b, cudaStream_t s) {
         if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_init, b->d_imgs + gr.offset, gr.count, gr.D, gInt, s);
     if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_set_counts, b->d_imgs, b->n, s);
     for (const auto& gr : b->groups)
-        if (e == cudaSuccess) e = mdas_launch_evaluate_batch(b->d_scenes + gr.offset, gr.count, gr.D, 1, gInt, s);
+        if (e == cudaSuccess) e = mdas_launch_evaluate_batch(b->d_scenes + gr.offset, gr.count, gr.D, gInt, s);
+    for (const auto& gr : b->groups)
+        if (e == cudaSuccess)
+            e = MDAS_ARITH_CALL(b, batch_initial_errors, b->d_imgs + gr.offset, gr.count, gr.D, b->numSMs * b->tune[0], s);
     return e;
 }
 
 cudaError_t enqueue_batch_body(mdas_batch* b, cudaGraphConditionalHandle handle, int* anyOut, cudaStream_t s) {
-    const int gErr = b->numSMs * b->tune[0], gDec = b->numSMs * b->tune[1], gPl = b->numSMs * b->tune[2];
-    const int gInt = b->numSMs * b->tune[3];
+    const int gDec = b->numSMs * b->tune[1], gPl = b->numSMs * b->tune[2], gVal = b->numSMs * b->tune[3];
     // (the accumulators of this pass were cleared by the last pass's scan, or
     // when the counters were set)
     // The dimensions' passes do not depend on one another: each dimension's chain
@@ -1127,7 +1123,6 @@ cudaError_t enqueue_batch_body(mdas_batch* b, cudaGraphConditionalHandle handle,
         const MdasBatchImage* imgs = b->d_imgs + gr.offset;
         const cudaStream_t gs = k == 0 ? s : b->groupStream[k];
         if (k > 0) e = cudaStreamWaitEvent(gs, b->forkEvent, 0);
-        if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_errors, imgs, gr.count, gr.D, gErr, gs);
         if (e == cudaSuccess && b->anyLearned) {
             // learned images: priorities of the leaves whose error was recomputed, then the judge
             e = MDAS_ARITH_CALL(b, batch_reset, imgs, gr.count, 2, gs);
@@ -1136,10 +1131,10 @@ cudaError_t enqueue_batch_body(mdas_batch* b, cudaGraphConditionalHandle handle,
         }
         if (e == cudaSuccess)
             e = MDAS_ARITH_CALL(b, batch_decide, imgs, gr.count, gr.D, b->tileK, b->anyLearned, gDec, gs);
-        if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_scan, imgs, gr.count, gs);
+        if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_scan, imgs, gr.count, kMaxGraphPasses, gs);
         if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_place, imgs, gr.count, gr.D, gPl, gs);
         if (e == cudaSuccess)
-            e = mdas_launch_evaluate_batch(b->d_scenes + gr.offset, gr.count, gr.D, 0, gInt, gs);
+            e = MDAS_ARITH_CALL(b, batch_values, imgs, b->d_scenes + gr.offset, gr.count, gr.D, gVal, gs);
         if (k > 0 && e == cudaSuccess) e = cudaEventRecord(b->joinEvent[k], gs);
     }
     for (size_t k = 1; k < b->groups.size() && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(s, b->joinEvent[k], 0);
@@ -1287,7 +1282,6 @@ int mdas_batch_create(mdas_batch** out, int n, mdas_grid* const* grids, mdas_sce
         bs.sc = scenes[i]->desc;
         bs.prims = scenes[i]->d_prims;
         bs.cull = scenes[i]->d_cull;
-        bs.counts = g->dg.counts;
         bs.coords = g->dg.coords;
         bs.values = g->dg.values;
         bs.dim = g->dg.D;

@@ -3,6 +3,7 @@
 
 #include <stdint.h>
 #include <cuda_runtime.h>
+#include "integrand.h"
 
 // Counters kept in device memory so that a pass never needs the host to know
 // how many leaves there are (the reference reads them back with
@@ -66,7 +67,8 @@ __host__ __device__ inline float mdas_float_unorder(unsigned u) {
 struct MdasCtl {
     int N0;
     int L0;
-    int pad[2];
+    int more;  // another pass of the render loop follows this one
+    int pad;
 };
 
 struct MdasDeviceGrid {
@@ -125,6 +127,17 @@ struct MdasBatchImage {
     const void* mlp;        // packed weights of a learned image (g.priority set), nullptr: plain acceptance
 };
 
+// The integrand side of one image of a batched render (device-side descriptor).
+struct MdasBatchScene {
+    MdasScene sc;
+    const float* prims;
+    const unsigned* cull;  // culling lists of the discs, or null
+    const float* coords;
+    float* values;
+    int dim;
+    int initialSamples;
+};
+
 // Leaves per thread and per tile of the adaptive pass (the default; the
 // batched renders may take 4 per thread: MdasDeviceGrid::tileK), and the
 // smallest tile, which sizes the per-tile scratch.
@@ -153,22 +166,24 @@ struct MdasBatchImage {
     cudaError_t pack_records(const MdasDeviceGrid& g, int L, const int* nodes, const float* boxes,          \
                              cudaStream_t s);                                                               \
     int record_floats(int D);                                                                               \
-    cudaError_t compute_errors_auto(const MdasDeviceGrid& g, int grid, cudaStream_t s);                     \
+    cudaError_t render_pass(const MdasDeviceGrid& g, const MdasScene& sc, const float* prims,               \
+                            const unsigned* cull, cudaGraphConditionalHandle h, int budget, int maxPasses,  \
+                            int gridDecide, int gridPlace, int gridValues, cudaStream_t s);                 \
     cudaError_t batch_init(const MdasBatchImage* imgs, int n, int D, int grid, cudaStream_t s);              \
     cudaError_t batch_set_counts(const MdasBatchImage* imgs, int n, cudaStream_t s);                         \
-    cudaError_t batch_errors(const MdasBatchImage* imgs, int n, int D, int grid, cudaStream_t s);            \
+    cudaError_t batch_initial_errors(const MdasBatchImage* imgs, int n, int D, int grid, cudaStream_t s);    \
+    cudaError_t batch_values(const MdasBatchImage* imgs, const MdasBatchScene* scenes, int n, int D,         \
+                             int grid, cudaStream_t s);                                                      \
     cudaError_t batch_reset(const MdasBatchImage* imgs, int n, int which, cudaStream_t s);                   \
     cudaError_t batch_decide(const MdasBatchImage* imgs, int n, int D, int K, bool learned, int grid,        \
                              cudaStream_t s);                                                                 \
-    cudaError_t batch_scan(const MdasBatchImage* imgs, int n, cudaStream_t s);                               \
+    cudaError_t batch_scan(const MdasBatchImage* imgs, int n, int maxPasses, cudaStream_t s);                \
     cudaError_t batch_place(const MdasBatchImage* imgs, int n, int D, int grid, cudaStream_t s);             \
     cudaError_t batch_condition(const MdasBatchImage* imgs, int n, cudaGraphConditionalHandle h,             \
                                 int maxPasses, int* anyOut, cudaStream_t s);                                 \
     cudaError_t batch_integrate(const MdasBatchImage* imgs, int n, int D, int grid, cudaStream_t s);         \
     cudaError_t batch_clear_pixels(const MdasBatchImage* imgs, int n, cudaStream_t s);                       \
     unsigned batch_jump(int candidatesNum, int D, unsigned* C);                                              \
-    cudaError_t loop_condition(const MdasDeviceGrid& g, cudaGraphConditionalHandle h, int budget,           \
-                               int maxPasses, cudaStream_t s);                                              \
     int max_blocks_per_sm(int D, int which);                                                                \
     cudaError_t learned_judge(const MdasDeviceGrid& g, int L, int grid, cudaStream_t s);                     \
     cudaError_t batch_learned_judge(const MdasBatchImage* imgs, int n, int grid, cudaStream_t s);            \
@@ -183,5 +198,6 @@ enum {
     MDAS_K_ADAPTIVE = 2,
     MDAS_K_INTEGRATE = 3,
     MDAS_K_DECIDE = 4,
-    MDAS_K_COUNT = 5
+    MDAS_K_RENDER_VALUES = 5,  // the new samples of a render loop's pass
+    MDAS_K_COUNT = 6
 };

@@ -114,20 +114,17 @@ __global__ void __launch_bounds__(256) k_evaluate(MdasScene sc, const float* __r
     }
 }
 
-// Batched integrand: chunks of 256 samples across the images of one launch
+// Batched integrand over the images' initial samples: chunks of 256 samples across
+// the images of one launch
 // (same enumeration scheme as the batched MDAS kernels); primitives are read
 // from global memory (L1/L2-resident), as several scenes share a launch.
 template <int D>
-__global__ void __launch_bounds__(256) k_evaluate_batch(const MdasBatchScene* __restrict__ scenes, int n, int all) {
+__global__ void __launch_bounds__(256) k_evaluate_batch(const MdasBatchScene* __restrict__ scenes, int n) {
     __shared__ int s_pre[257];
     __shared__ unsigned s_warp[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned v = 0;
-    if (threadIdx.x < (unsigned)n) {
-        const MdasCounts* c = scenes[threadIdx.x].counts;
-        const int items = all ? scenes[threadIdx.x].initialSamples : (c->active ? c->newN : 0);
-        v = (unsigned)((items + 255) / 256);
-    }
+    if (threadIdx.x < (unsigned)n) v = (unsigned)((scenes[threadIdx.x].initialSamples + 255) / 256);
     unsigned incl = v;
     for (int o = 1; o < 32; o <<= 1) {
         const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -156,11 +153,9 @@ __global__ void __launch_bounds__(256) k_evaluate_batch(const MdasBatchScene* __
             else hi = mid - 1;
         }
         const MdasBatchScene& b = scenes[lo];
-        const int offset = all ? 0 : b.counts->N - b.counts->newN;
-        const int count = all ? b.initialSamples : b.counts->newN;
         const int k = (ch - s_pre[lo]) * 256 + threadIdx.x;
-        if (k < count) {
-            const size_t s = (size_t)offset + k;
+        if (k < b.initialSamples) {
+            const size_t s = (size_t)k;
             float c[D];
 #pragma unroll
             for (int d = 0; d < D; ++d) c[d] = b.coords[s * D + d];
@@ -426,12 +421,12 @@ cudaError_t mdas_launch_evaluate(const MdasScene& sc, const float* d_prims, cons
     return cudaGetLastError();
 }
 
-cudaError_t mdas_launch_evaluate_batch(const MdasBatchScene* scenes, int n, int D, int all, int grid, cudaStream_t s) {
+cudaError_t mdas_launch_evaluate_batch(const MdasBatchScene* scenes, int n, int D, int grid, cudaStream_t s) {
     switch (D) {
-        case 3: k_evaluate_batch<3><<<grid, 256, 0, s>>>(scenes, n, all); break;
-        case 4: k_evaluate_batch<4><<<grid, 256, 0, s>>>(scenes, n, all); break;
-        case 5: k_evaluate_batch<5><<<grid, 256, 0, s>>>(scenes, n, all); break;
-        case 6: k_evaluate_batch<6><<<grid, 256, 0, s>>>(scenes, n, all); break;
+        case 3: k_evaluate_batch<3><<<grid, 256, 0, s>>>(scenes, n); break;
+        case 4: k_evaluate_batch<4><<<grid, 256, 0, s>>>(scenes, n); break;
+        case 5: k_evaluate_batch<5><<<grid, 256, 0, s>>>(scenes, n); break;
+        case 6: k_evaluate_batch<6><<<grid, 256, 0, s>>>(scenes, n); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -38,6 +38,7 @@
 #include "ieee_math.h"
 #include "leaf_raw.h"
 #include "ld_hint.h"
+#include "shade.cuh"
 
 #ifndef MDAS_NS
 #error "define MDAS_NS before including kdgrid_kernels.cuh"
@@ -314,24 +315,21 @@ __global__ void __launch_bounds__(256) k_initial_sampling(MdasDeviceGrid g, int 
 //           slot range [L - newL, L)); the max over all other leaves was taken
 //           by the adaptive pass that left them unchanged (counts->gerrNext).
 // =====================================================================================
-// The error of a leaf with sample list `node` and box volume `volume`; lumOut
-// (may be null) receives the luminance statistics of its samples.
-template <int D>
-__device__ __forceinline__ float node_error(const MdasDeviceGrid& g, const int4 node, const float volume,
-                                            MdasLumStats* lumOut) {
+// The error of a leaf with the values loc of the samples in its filled slots
+// (bits of `filled`, sampleCount of them) and box volume `volume`; lumOut (may be
+// null) receives the luminance statistics of its samples.  (sampleCount is not a
+// compile-time constant in any caller: its reciprocal is the hardware's in the
+// reference's arithmetic.)
+__device__ __forceinline__ float values_error(const float3 (&loc)[4], unsigned filled, int sampleCount,
+                                              const float volume, MdasLumStats* lumOut) {
     float3 avg = make_float3(0.0f, 0.0f, 0.0f);
-    float3 loc[4];
-    int sampleCount = 0;
     MdasLumStats lum = mdas_lum_empty();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int idx = node_get(node, i);
-        if (idx >= 0) {
-            loc[i] = ld_value64(g.values, idx);
+        if ((filled >> i) & 1u) {
             avg.x += loc[i].x;
             avg.y += loc[i].y;
             avg.z += loc[i].z;
-            sampleCount++;
             if (lumOut) mdas_lum_add(lum, mdas_luminance(loc[i].x, loc[i].y, loc[i].z));
         }
     }
@@ -362,6 +360,23 @@ __device__ __forceinline__ float node_error(const MdasDeviceGrid& g, const int4 
     return error;
 }
 
+// The error of a leaf with sample list `node`.
+template <int D>
+__device__ __forceinline__ float node_error(const MdasDeviceGrid& g, const int4 node, const float volume,
+                                            MdasLumStats* lumOut) {
+    float3 loc[4];
+    unsigned filled = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int idx = node_get(node, i);
+        if (idx >= 0) {
+            loc[i] = ld_value64(g.values, idx);
+            filled |= 1u << i;
+        }
+    }
+    return values_error(loc, filled, __popc(filled), volume, lumOut);
+}
+
 template <int D>
 __device__ __forceinline__ float leaf_error(const MdasDeviceGrid& g, int nodeIndex) {
     float mn[D], mx[D];
@@ -369,14 +384,15 @@ __device__ __forceinline__ float leaf_error(const MdasDeviceGrid& g, int nodeInd
     return node_error<D>(g, node, box_volume<D>(mn, mx), nullptr);
 }
 
-// MODE 0: full, 1: dirty, 2: dirty unless no adaptive pass ran since the
-// initial sampling (the device-side budget loop, where passes alternate).
+// (The device-side render loops compute the errors of split children with the new
+// samples' values, in k_render_values.)
+// MODE 0: full, 1: dirty.
 template <int D, int MODE>
 __global__ void __launch_bounds__(256, 6) k_compute_errors(MdasDeviceGrid g) {
     pdl_launch_dependents();  // decide may be scheduled; it waits for this grid
     __shared__ unsigned s_max[8];
     __shared__ unsigned s_cnt[8];
-    const bool DIRTY = MODE == 1 || (MODE == 2 && g.counts->passes > 0);
+    constexpr bool DIRTY = MODE == 1;
     int items, newL = 0, firstRight = 0;
     float maxError = 0.0f;
     if (DIRTY) {
@@ -721,7 +737,12 @@ __global__ void __launch_bounds__(256, LEARNED ? 1 : 4) k_adaptive_decide(MdasDe
 
 // One CTA of 1024 threads: exclusive prefix over the tile counts, then the
 // counters (N, L as the place kernel must see them go to ctl).
-__device__ __forceinline__ void scan_image(const MdasDeviceGrid& g, unsigned* s_sel, unsigned* s_split) {
+// Returns, to the thread that set the counters (the last one), whether another
+// pass follows this one in a render loop over `budget` samples: N < budget, the
+// next pass fits, no device error and fewer than maxPasses passes ran
+// (optixMotionBlur.cpp:781, 723-724); the verdict also goes to ctl->more.
+__device__ __forceinline__ bool scan_image(const MdasDeviceGrid& g, unsigned* s_sel, unsigned* s_split, int budget,
+                                           int maxPasses) {
     const int N = g.counts->N;
     const int L = g.counts->L;
     const int tileLeaves = 256 * g.tileK;
@@ -796,15 +817,31 @@ __device__ __forceinline__ void scan_image(const MdasDeviceGrid& g, unsigned* s_
         c->recomputed = 0;
         c->gathered = 0u;
         c->gerrNext = 0u;
-        c->passes += 1;
+        const int passes = c->passes + 1;
+        c->passes = passes;
+        const long long N1 = (long long)N + (int)newN, L1 = (long long)L + (int)newL;
+        const bool more = N1 < budget && N1 + L1 <= g.maxSamples && c->status == 0 && passes < maxPasses;
+        g.ctl->more = more ? 1 : 0;
+        return more;
     }
+    return false;
 }
 
 __global__ void __launch_bounds__(1024) k_adaptive_scan(MdasDeviceGrid g) {
     pdl_wait();
     pdl_launch_dependents();
     __shared__ unsigned s_sel[32], s_split[32];
-    scan_image(g, s_sel, s_split);
+    scan_image(g, s_sel, s_split, 0, 0);
+}
+
+// The scan of the device-side render loop: also sets the loop's condition.
+__global__ void __launch_bounds__(1024) k_loop_scan(MdasDeviceGrid g, cudaGraphConditionalHandle h, int budget,
+                                                    int maxPasses) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ unsigned s_sel[32], s_split[32];
+    const bool more = scan_image(g, s_sel, s_split, budget, maxPasses);
+    if (threadIdx.x == 1023) cudaGraphSetConditional(h, more ? 1u : 0u);
 }
 
 // 16-byte chunks of a leaf record that the adaptive pass reads (node, box, padding, private copy)
@@ -1010,9 +1047,12 @@ __device__ __forceinline__ void store_split_lists(const MdasDeviceGrid& g, const
 // scalar stores per split): 5-D 1920x1080 frame at 32 spp 15.96 -> 13.26 ms,
 // learned at 16 spp 8.96 -> 7.78 ms, 4-D 1024x1024 at 16 spp 2.539 -> 2.515 ms,
 // 4-D 4K at 16 spp 23.9 -> 23.4 ms (whole frames).
+//
+// render: the pass belongs to a render loop; each new sample's split rank (-1: an
+// append) is left where its group's values will be, for k_render_values.
 template <int D>
 __device__ __forceinline__ void place_warp(const MdasDeviceGrid& g, int tile, uint2 pre, uint2 e, int N, int L, int kb,
-                                           int count, float4* slots, float* newPoints) {
+                                           int count, float4* slots, float* newPoints, bool render) {
     constexpr int NB = NbLayout<D>::FLOATS, SC = NbLayout<D>::SC;
     constexpr int C = RecChunks<D>::C, CS = RecChunks<D>::CS;
     const int lane = threadIdx.x & 31;
@@ -1100,10 +1140,11 @@ __device__ __forceinline__ void place_warp(const MdasDeviceGrid& g, int tile, ui
                 *reinterpret_cast<float4*>(g.nb + (size_t)leaf * NB + 4 * c) = slots[r * CS + c];
         }
     }
+    const int rank = (int)pre.y + (int)((e.x >> 11) & 0x7ffu);
+    if (render && active) g.values[3 * (size_t)(N + kb) + lane] = __int_as_float(split ? rank : -1);
     const unsigned splits = __ballot_sync(0xffffffffu, split);
     if (splits) {
         __syncwarp();  // every lane's record is read: the slots take the right children
-        const int rank = (int)pre.y + (int)((e.x >> 11) & 0x7ffu);
         const int rank0 = __shfl_sync(0xffffffffu, rank, __ffs(splits) - 1);
         if (split) {
             float4* out = slots + __popc(splits & ((1u << lane) - 1u)) * CS;
@@ -1225,7 +1266,7 @@ __device__ __forceinline__ void warp_locate(const MdasDeviceGrid& g, int kb, int
 // against one thread per leaf loading its record when its turn comes: adaptive
 // stage -4 % on dof1024, -18 % on mbdof1080.
 template <int D>
-__global__ void __launch_bounds__(256, D >= 5 ? 2 : 3) k_adaptive_place(MdasDeviceGrid g) {
+__global__ void __launch_bounds__(256, D >= 5 ? 2 : 3) k_adaptive_place(MdasDeviceGrid g, bool render) {
     constexpr int CS = RecChunks<D>::CS;
     __shared__ __align__(16) float4 s_rec[2][8][32 * CS];
     __shared__ float s_new[D == 4 ? 1 : 8][D == 4 ? 1 : 32 * D];  // the warps' new points (place_warp)
@@ -1267,7 +1308,7 @@ __global__ void __launch_bounds__(256, D >= 5 ? 2 : 3) k_adaptive_place(MdasDevi
         }
         __syncwarp();
         place_warp<D>(g, tile0, pre0, e0, N, L, kb, min(32, accepted - kb), s_rec[buf][warp],
-                      s_new[D == 4 ? 0 : warp]);
+                      s_new[D == 4 ? 0 : warp], render);
         __syncwarp();  // the buffer is refilled two iterations on
         if (!more) break;
         e0 = e1;
@@ -1275,6 +1316,106 @@ __global__ void __launch_bounds__(256, D >= 5 ? 2 : 3) k_adaptive_place(MdasDevi
         pre0 = pre1;
         kb = kn;
         buf ^= 1;
+    }
+}
+
+// =====================================================================================
+// The pass's new samples in a render loop: their values, and the errors of the
+// split children, in one kernel.
+//
+// The drop-in calls leave the values to the caller and the errors to the next
+// errors pass; a render loop evaluates the samples itself, so the two kernels after
+// place become one: a split's old values are gathered while its new sample is
+// evaluated, that sample's value is not gathered at all, and a pass has two
+// launches less (with the loop's condition in the scan).  After the last pass the
+// children stay as an adaptive pass leaves them (error -1, listed for an errors
+// pass).
+//
+// Latency bounds it (gathers of 64 DRAM bytes at random, chains of list and disc
+// loads): 3-D 256x256 frame at 8 spp (29 passes) 0.633 -> 0.561 ms, 5-D 1920x1080
+// at 32 spp 12.36 -> 12.17 ms, 4-D 1024x1024 2.281 -> 2.268 ms, 12-image batch
+// 41.9 -> 41.8 ms.  Measured and slower: the children of a 256-sample chunk spread
+// over its threads with block barriers (0.640 ms, 12.36 ms, 2.39 ms), 3 or 5 CTAs
+// per SM, place letting this kernel start before it ends (12-15 % slower frames).
+// =====================================================================================
+// The sample of rank k (its group's warp calls this together; k >= accepted: a lane
+// without one).  Returns the larger error of its children (0 without).
+template <int D>
+__device__ __forceinline__ float render_sample(const MdasDeviceGrid& g, const MdasScene& sc,
+                                               const float* __restrict__ prims, const unsigned* __restrict__ cull, int k,
+                                               int accepted, int N, int L, bool more) {
+    const bool active = k < accepted;
+    const size_t s = (size_t)N + k;
+    float c[D];
+    int rank = -1;
+    if (active) {
+        rank = __float_as_int(g.values[3 * ((size_t)N + (k & ~31)) + (k & 31)]);  // (place_warp's note)
+#pragma unroll
+        for (int d = 0; d < D; ++d) c[d] = g.coords[s * D + d];
+    }
+    const bool split = active && more && rank >= 0;
+    int4 l = make_int4(0, 0, 0, 0), r = l;
+    float3 v[5];
+    if (split) {
+        l = g.splitL[rank];
+        r = g.splitR[rank];
+        const int idx[5] = {l.x, l.y, r.x, r.y, r.z};
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+            if (idx[i] != N + k) v[i] = ld_value64(g.values, idx[i]);
+    }
+    float val[3] = {0.0f, 0.0f, 0.0f};
+    if (active) {
+        if (cull) shade_culled(sc, prims, cull, c, val);
+        else mdas_shade(&sc, prims, c, val);
+    }
+    __syncwarp();  // the group's notes are read: its values may take their place
+    if (active) {
+        g.values[3 * s + 0] = val[0];
+        g.values[3 * s + 1] = val[1];
+        g.values[3 * s + 2] = val[2];
+    }
+    if (!split) return 0.0f;
+    const int idx[5] = {l.x, l.y, r.x, r.y, r.z};
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+        if (idx[i] == N + k) v[i] = make_float3(val[0], val[1], val[2]);
+    const float3 z = make_float3(0.0f, 0.0f, 0.0f);
+    const float3 lv[4] = {v[0], v[1], z, z}, rv[4] = {v[2], v[3], v[4], z};
+    int n2 = 2, n3 = 3;
+    asm volatile("" : "+r"(n2), "+r"(n3));  // not constants to the compiler (values_error)
+    MdasLumStats lum;
+    const float errL = values_error(lv, 3u, n2, __int_as_float(l.w), g.featRaw ? &lum : nullptr);
+    if (g.featRaw) mdas_raw_store_stats(g.featRaw + (size_t)rank * MDAS_RAW_FLOATS, lum, errL);
+    const float errR = values_error(rv, 7u, n3, __int_as_float(r.w), g.featRaw ? &lum : nullptr);
+    if (g.featRaw) mdas_raw_store_stats(g.featRaw + (size_t)(g.counts->newL + rank) * MDAS_RAW_FLOATS, lum, errR);
+    g.errors[l.z] = errL;
+    g.errors[L + rank] = errR;
+    return fmaxf(errL, errR);
+}
+
+template <int D>
+__global__ void __launch_bounds__(256, 4) k_render_values(MdasDeviceGrid g, const __grid_constant__ MdasScene sc,
+                                                       const float* __restrict__ prims,
+                                                       const unsigned* __restrict__ cull) {
+    __shared__ unsigned s_max[8];
+    pdl_wait();
+    const int N = g.ctl->N0, L = g.ctl->L0, accepted = g.counts->newN;
+    const bool more = g.ctl->more != 0;
+    float maxError = 0.0f;
+    for (int base = blockIdx.x * 256; base < accepted; base += gridDim.x * 256)
+        maxError = fmaxf(maxError, render_sample<D>(g, sc, prims, cull, base + threadIdx.x, accepted, N, L, more));
+    if (!more) return;
+    // g_error for the next pass: over the children and the leaves the pass kept
+    // (kdgrid.cu:684-716 takes it over all leaves)
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(maxError));
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned b = blockIdx.x == 0 ? g.counts->gerrCarry : 0u;
+        for (int k = 0; k < 8; ++k) b = max(b, s_max[k]);
+        if (b) atomicMax(&g.counts->gerr, b);
+        if (blockIdx.x == 0) g.counts->recomputed = 2 * g.counts->newL;
     }
 }
 
@@ -1571,7 +1712,7 @@ __global__ void __launch_bounds__(256) k_learned_judge(MdasDeviceGrid g, int Lho
 // A launch that may overlap the tail of the previous kernel on the stream (the
 // kernel calls pdl_wait() before it reads what that kernel wrote).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args... args) {
+cudaError_t launch_on(void (*kernel)(KArgs...), bool dependent, int grid, int block, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
@@ -1581,8 +1722,13 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args... args) {
+    return launch_on(kernel, true, grid, block, s, args...);
 }
 
 #define MDAS_SWITCH_D(D, EXPR)                 \
@@ -1612,28 +1758,6 @@ cudaError_t compute_errors(const MdasDeviceGrid& g, int grid, bool dirty, cudaSt
     return cudaGetLastError();
 }
 
-cudaError_t compute_errors_auto(const MdasDeviceGrid& g, int grid, cudaStream_t s) {
-    MDAS_SWITCH_D(g.D, (k_compute_errors<DD, 2><<<grid, 256, 0, s>>>(g)));
-    return cudaGetLastError();
-}
-
-// Condition of the device-side budget loop (optixMotionBlur.cpp:781 plus the
-// capacity guard of :723-724): another pass while N < budget, the next pass
-// fits, no device error, and fewer than maxPasses passes ran (a safety stop:
-// every pass accepts at least the leaf with the largest error, so N grows).
-__global__ void k_loop_condition(const MdasCounts* __restrict__ c, cudaGraphConditionalHandle h, int budget,
-                                 int maxSamples, int maxPasses) {
-    const long long N = c->N, L = c->L;
-    cudaGraphSetConditional(h, (N < budget && N + L <= maxSamples && c->status == 0 && c->passes < maxPasses) ? 1u
-                                                                                                             : 0u);
-}
-
-cudaError_t loop_condition(const MdasDeviceGrid& g, cudaGraphConditionalHandle h, int budget, int maxPasses,
-                           cudaStream_t s) {
-    k_loop_condition<<<1, 1, 0, s>>>(g.counts, h, budget, g.maxSamples, maxPasses);
-    return cudaGetLastError();
-}
-
 // LCG jump-ahead: n draws take a seed s to A_n * s + C_n (mod 2^32).
 static void lcg_jump(unsigned n, unsigned* A, unsigned* C) {
     unsigned a = 1u, c = 0u;
@@ -1660,27 +1784,50 @@ static cudaError_t place_prepare(int D) {
     return e;
 }
 
-cudaError_t adaptive_sampling(const MdasDeviceGrid& g, int gridDecide, int gridPlace, cudaStream_t s) {
+// dependent: programmatic dependence on the kernel before it on the stream.
+static cudaError_t launch_decide(const MdasDeviceGrid& g, bool dependent, int grid, cudaStream_t s) {
     cudaError_t e = cudaSuccess;
     unsigned A, C;
     lcg_jump((unsigned)(g.candidatesNum * g.D), &A, &C);
     if (g.priority && g.tileK == 4) {
-        MDAS_SWITCH_D(g.D, (e = launch_pdl(k_adaptive_decide<DD, 4, true>, gridDecide, 256, s, g, A, C)));
+        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 4, true>, dependent, grid, 256, s, g, A, C)));
     } else if (g.priority) {
-        MDAS_SWITCH_D(g.D, (e = launch_pdl(k_adaptive_decide<DD, 8, true>, gridDecide, 256, s, g, A, C)));
+        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 8, true>, dependent, grid, 256, s, g, A, C)));
     } else if (g.tileK == 4) {
-        MDAS_SWITCH_D(g.D, (e = launch_pdl(k_adaptive_decide<DD, 4, false>, gridDecide, 256, s, g, A, C)));
+        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 4, false>, dependent, grid, 256, s, g, A, C)));
     } else {
-        MDAS_SWITCH_D(g.D, (e = launch_pdl(k_adaptive_decide<DD, 8, false>, gridDecide, 256, s, g, A, C)));
+        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 8, false>, dependent, grid, 256, s, g, A, C)));
     }
+    return e;
+}
+
+static cudaError_t launch_place(const MdasDeviceGrid& g, bool render, int grid, cudaStream_t s) {
+    cudaError_t e = place_prepare(g.D);
     if (e != cudaSuccess) return e;
-    e = launch_pdl(k_adaptive_scan, 1, 1024, s, g);
-    if (e != cudaSuccess) return e;
-    e = place_prepare(g.D);
-    if (e != cudaSuccess) return e;
-    MDAS_SWITCH_D(g.D, (e = launch_pdl(k_adaptive_place<DD>, gridPlace, 256, s, g)));
-    if (e != cudaSuccess) return e;
-    return cudaGetLastError();
+    MDAS_SWITCH_D(g.D, (e = launch_pdl(k_adaptive_place<DD>, grid, 256, s, g, render)));
+    return e;
+}
+
+cudaError_t adaptive_sampling(const MdasDeviceGrid& g, int gridDecide, int gridPlace, cudaStream_t s) {
+    cudaError_t e = launch_decide(g, true, gridDecide, s);
+    if (e == cudaSuccess) e = launch_pdl(k_adaptive_scan, 1, 1024, s, g);
+    if (e == cudaSuccess) e = launch_place(g, false, gridPlace, s);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+// One pass of the device-side render loop (the leaf errors are current): decide, the
+// scan with the loop's condition, place, and the new samples' values with the errors
+// of the split children.
+cudaError_t render_pass(const MdasDeviceGrid& g, const MdasScene& sc, const float* prims, const unsigned* cull,
+                        cudaGraphConditionalHandle h, int budget, int maxPasses, int gridDecide, int gridPlace,
+                        int gridValues, cudaStream_t s) {
+    // (decide is the loop body's first kernel unless the learned judge comes before it)
+    cudaError_t e = launch_decide(g, g.priority != nullptr, gridDecide, s);
+    if (e == cudaSuccess) e = launch_pdl(k_loop_scan, 1, 1024, s, g, h, budget, maxPasses);
+    if (e == cudaSuccess) e = launch_place(g, true, gridPlace, s);
+    if (e == cudaSuccess)
+        MDAS_SWITCH_D(g.D, (e = launch_pdl(k_render_values<DD>, gridValues, 256, s, g, sc, prims, cull)));
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t learned_judge(const MdasDeviceGrid& g, int L, int grid, cudaStream_t s) {
@@ -1753,6 +1900,9 @@ int max_blocks_per_sm(int D, int which) {
             break;
         case MDAS_K_INTEGRATE:
             MDAS_SWITCH_D(D, (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_integrate<DD>, 256, 0)));
+            break;
+        case MDAS_K_RENDER_VALUES:
+            MDAS_SWITCH_D(D, (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_render_values<DD>, 256, 0)));
             break;
         case MDAS_K_DECIDE:
             MDAS_SWITCH_D(D, (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adaptive_decide<DD, 8, false>,

@@ -33,22 +33,9 @@ cudaError_t mdas_launch_reference_image(const MdasScene& sc, const float* d_prim
 int mdas_generate_scene(int kind, uint64_t seed, int count, float scaleX, float scaleY, int width, int height,
                         MdasScene* sc, std::vector<float>* prims);
 
-// The integrand side of one image of a batched render (device-side descriptor).
-struct MdasBatchScene {
-    MdasScene sc;
-    const float* prims;
-    const unsigned* cull;  // culling lists of the discs, or null
-    const MdasCounts* counts;
-    const float* coords;
-    float* values;
-    int dim;
-    int initialSamples;
-};
-
-// Batched integrand: every image's initial samples (all = 1) or the samples the
-// last pass added to each still-active image (all = 0).  Images of one launch
+// Batched integrand over every image's initial samples.  Images of one launch
 // share the coordinate stride D.
-cudaError_t mdas_launch_evaluate_batch(const MdasBatchScene* scenes, int n, int D, int all, int grid, cudaStream_t s);
+cudaError_t mdas_launch_evaluate_batch(const MdasBatchScene* scenes, int n, int D, int grid, cudaStream_t s);
 
 struct mdas_scene {
     MdasScene desc;
