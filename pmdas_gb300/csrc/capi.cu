@@ -93,7 +93,7 @@ struct mdas_grid {
     int2* hChildren = nullptr;        // [cap] children of the internal nodes
     int* hParents = nullptr;          // [2 cap] parents of the internal nodes, then of the leaves
     float* hBoxes = nullptr;          // [cap * 2D] boxes of the internal nodes
-    unsigned* hVisits = nullptr;      // [cap + 1] refit arrival counters, then the locate status word
+    unsigned* hVisits = nullptr;      // [cap + 1] meeting points of the tree's construction, then the locate status word
     void* sortTemp = nullptr;
     size_t sortTempBytes = 0;
     // point location: coarse keys of the queries (2 cap), their order, sort scratch
@@ -1657,9 +1657,10 @@ int mdas_build_hierarchy(mdas_grid* g, int fineBits) {
     int rc = order_leaves(g, fineBits);
     if (rc) return rc;
     const int n = g->L;
-    cudaError_t e = mdas_order::karras_build(g->hSorted, n, g->hChildren, g->hParents, g->stream);
-    if (e == cudaSuccess)
-        e = mdas_order::karras_refit(g->dg, g->hOrder, n, g->hChildren, g->hParents, g->hVisits, g->hBoxes, g->stream);
+    // (the sort is done with its scratch)
+    if (mdas_order::tree_scratch_bytes(n) > g->sortTempBytes) return MDAS_ERR_INVALID;
+    cudaError_t e = mdas_order::karras_tree(g->dg, g->hSorted, g->hOrder, n, g->hChildren, g->hParents, g->hVisits,
+                                            g->sortTemp, g->hBoxes, g->stream);
     g->launches += 2;
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     if (e != cudaSuccess) return MDAS_ERR_CUDA;

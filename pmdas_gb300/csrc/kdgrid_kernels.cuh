@@ -1490,25 +1490,17 @@ __device__ __forceinline__ void integrate_leaf(const MdasDeviceGrid& g, const in
     }
 }
 
-// Node and box of the 32 consecutive leaves [first, first + 32), read by the
-// warp into shared memory with each 16-byte load covering consecutive record
-// heads (a third of the lines that 32 lanes each reading their own record
-// touch, the records being a 128-byte line apart at D = 4), then this lane's
-// from there.  Every lane of the warp calls it; false past the last leaf.
+// Node and box of this lane's leaf of the 32 consecutive ones [first, first + 32),
+// read by the warp together.  Every lane of the warp calls it; false past the last
+// leaf.
 template <int D>
 __device__ __forceinline__ bool warp_leaf_head(const float* __restrict__ nb, int first, int L, float4* wbuf,
                                                int4& node, float (&mn)[D], float (&mx)[D]) {
     constexpr int H4 = (4 + 2 * D + 3) / 4;  // 16-byte chunks of node + box
     constexpr int NB = NbLayout<D>::FLOATS;
     static_assert(4 * H4 <= NB, "the chunks stay inside the record");
+    warp_heads64<H4>(nb, NB, first, L, wbuf);
     const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int q = 0; q < H4; ++q) {
-        const int c = q * 32 + lane;
-        const int rec = c / H4;
-        if (first + rec < L) wbuf[c] = ld4_hint<64>(nb + (size_t)(first + rec) * NB + 4 * (c - rec * H4));
-    }
-    __syncwarp();
     const bool valid = first + lane < L;
     if (valid) {
         const float* h = reinterpret_cast<const float*>(wbuf + lane * H4);

@@ -55,3 +55,20 @@ __device__ __forceinline__ void ld_head64(const float* p, float (&out)[(NF + 3) 
         out[4 * k + 3] = v.w;
     }
 }
+
+// The first H4 16-byte chunks of the 32 consecutive records [first, first + 32) (of
+// L; `stride` floats apart), read by the warp into wbuf (record r's at wbuf + r * H4)
+// with each load covering consecutive chunks: a third of the lines that 32 lanes
+// each reading their own record touch.
+template <int H4>
+__device__ __forceinline__ void warp_heads64(const float* __restrict__ nb, size_t stride, int first, int L,
+                                             float4* wbuf) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < H4; ++q) {
+        const int c = q * 32 + lane;
+        const int rec = c / H4;
+        if (first + rec < L) wbuf[c] = ld4_hint<64>(nb + (size_t)(first + rec) * stride + 4 * (c - rec * H4));
+    }
+    __syncwarp();
+}

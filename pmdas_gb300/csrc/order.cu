@@ -72,10 +72,14 @@ __device__ __forceinline__ uint64_t spread_two(uint32_t x) {
 // axes go to bit D * K + 2 (b - K) + 1 - j (the initial-cell numbering of
 // uniformSamplingKernel, kdgrid.cu:144-160, extended to K bits).  `spread`:
 // spread_byte(v, D) for v < 256.
+// DIM: k.D where it is known at compile time (0: not known).
+template <int DIM = 0>
 __device__ __forceinline__ uint64_t point_key(const float* p, const KeyParams& k, const uint64_t* spread) {
     uint64_t key = 0;
     const uint32_t lowMask = k.K >= 32 ? 0xffffffffu : ((1u << k.K) - 1u);
-    for (int j = 0; j < k.D; ++j) {
+    const int D = DIM ? DIM : k.D;
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
         float u = p[j];
         if (j == 0) u = __fdiv_rn(u, k.scaleX);
         if (j == 1) u = __fdiv_rn(u, k.scaleY);
@@ -83,8 +87,8 @@ __device__ __forceinline__ uint64_t point_key(const float* p, const KeyParams& k
         const uint32_t q = quantize(u, B);
         const uint32_t low = q & lowMask;
         for (int m = 0; 8 * m < k.K; ++m)
-            key |= spread[(low >> (8 * m)) & 0xffu] << (k.D * 8 * m + (k.D - 1 - j));
-        if (j < 2 && k.eib > 0) key |= spread_two(q >> k.K) << (k.D * k.K + 1 - j);
+            key |= spread[(low >> (8 * m)) & 0xffu] << (D * 8 * m + (D - 1 - j));
+        if (j < 2 && k.eib > 0) key |= spread_two(q >> k.K) << (D * k.K + 1 - j);
     }
     return key;
 }
@@ -130,24 +134,40 @@ __global__ void k_morton_decode(const uint64_t* __restrict__ cells, int n, KeyPa
     }
 }
 
+// The records' heads are read by whole warps (ld_hint.h): each lane reading its own
+// touched a line or two per load and lane.  5.9 M leaves at D = 4: 115 -> 80 us.
 template <int D>
-__global__ void k_leaf_keys(const float* __restrict__ nb, int nbFloats, int L, KeyParams kp,
-                            uint64_t* __restrict__ keys) {
+__global__ void __launch_bounds__(256) k_leaf_keys(const float* __restrict__ nb, int nbFloats, int L, KeyParams kp,
+                                                   uint64_t* __restrict__ keys) {
+    constexpr int H4 = (4 + 2 * D + 3) / 4;
     __shared__ uint64_t s_spread[256];
+    __shared__ float4 s_head[8][32 * H4];
     load_spread(s_spread, kp.D);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L; i += gridDim.x * blockDim.x) {
-        float h[(4 + 2 * D + 3) / 4 * 4];  // node and box of the record (it extends past them)
-        ld_head64<4 + 2 * D>(nb + (size_t)i * nbFloats, h);
-        float c[D];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int base = blockIdx.x * 256; base < L; base += gridDim.x * 256) {
+        const int first = base + 32 * warp;
+        warp_heads64<H4>(nb, nbFloats, first, L, s_head[warp]);
+        if (first + lane < L) {
+            const float* h = reinterpret_cast<const float*>(s_head[warp] + lane * H4);
+            float c[D];
 #pragma unroll
-        for (int j = 0; j < D; ++j) c[j] = __fmul_rn(0.5f, __fadd_rn(h[4 + j], h[4 + D + j]));
-        keys[i] = point_key(c, kp, s_spread);
+            for (int j = 0; j < D; ++j) c[j] = __fmul_rn(0.5f, __fadd_rn(h[4 + j], h[4 + D + j]));
+            keys[first + lane] = point_key<D>(c, kp, s_spread);
+        }
+        __syncwarp();  // the buffer is refilled
     }
 }
 
 static int blocks_for(int n, int threads) {
     const int b = (n + threads - 1) / threads;
     return b < 1 ? 1 : (b > 65535 * 4 ? 65535 * 4 : b);
+}
+
+static int sm_count() {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 1;
 }
 
 cudaError_t morton_encode(const float* points, int n, int D, int bpd, int eib, int F, float sx, float sy,
@@ -178,7 +198,7 @@ cudaError_t morton_decode(const uint64_t* cells, int n, int D, int bpd, int eib,
 cudaError_t leaf_keys(const MdasDeviceGrid& g, int L, int F, uint64_t* keys, cudaStream_t s) {
     if (L <= 0) return cudaSuccess;
     const KeyParams kp{g.D, g.bitsPerDim + F, g.extraImgBits, g.scaleX, g.scaleY};
-    ORDER_SWITCH_D(g.D, (k_leaf_keys<DD><<<blocks_for(L, 256), 256, 0, s>>>(g.nb, g.nbFloats, L, kp, keys)));
+    ORDER_SWITCH_D(g.D, (k_leaf_keys<DD><<<min(blocks_for(L, 256), 8 * sm_count()), 256, 0, s>>>(g.nb, g.nbFloats, L, kp, keys)));
     return cudaGetLastError();
 }
 
@@ -495,14 +515,11 @@ cudaError_t radix_sort(void* temp, size_t tempBytes, const uint64_t* keysIn, uin
         k_iota<<<blocks_for(n, 256), 256, 0, s>>>(valuesOut, n);
         return cudaGetLastError();
     }
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (kSweepSmem > 0) {
         e = cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem);
         if (e != cudaSuccess) return e;
     }
-    const int histBlocks = min(blocks_for(n, kThreads), 2 * (sms > 0 ? sms : 1));
+    const int histBlocks = min(blocks_for(n, kThreads), 2 * sm_count());
     k_histogram<<<histBlocks, kThreads, 0, s>>>(keysIn, n, beginBit, endBit, passes, hist);
     k_digit_starts<<<passes, kBins, 0, s>>>(hist);
     const size_t tiles = ((size_t)n + kTile - 1) / kTile;
@@ -535,65 +552,50 @@ cudaError_t radix_sort(void* temp, size_t tempBytes, const uint64_t* keysIn, uin
 
 // ---------------------------------------------------------------------------------
 // Karras radix tree (T. Karras, "Maximizing Parallelism in the Construction of
-// BVHs, Octrees, and k-d Trees", HPG 2012): one thread per internal node finds
-// its key range from common-prefix lengths and splits it at the highest
-// differing bit.  Equal keys are told apart by their positions (the prefix
-// length of two equal keys is 64 + the common prefix of their positions).
+// BVHs, Octrees, and k-d Trees", HPG 2012) over the sorted keys, with the boxes of
+// its nodes.  Equal keys are told apart by their positions (the prefix length of two
+// equal keys is 64 + the common prefix of their positions).
+//
+// Built bottom-up (the pairing of C. Apetrei, "Fast and Simple Agglomerative LBVH
+// Construction", CGVC 2014): a subtree over the positions [l, r] belongs with the
+// neighbour whose key shares the longer prefix with its end, so its parent splits
+// at gamma = r (it is the left child) or gamma = l - 1 (the right one).  The two
+// children of a split meet at gamma: the first leaves its far end there and stops,
+// the second joins both.  Karras numbers the node over [l, r] r if it is a left
+// child and l if it is a right one (the root 0), so that the children of the split
+// gamma are gamma and gamma + 1; node numbers, children and parents are the ones
+// of his top-down construction.
+//
+// A CTA takes kRun consecutive positions and joins everything inside them in shared
+// memory: in rounds over a queue of the subtrees that still climb (half of them end
+// in each round; threads that climb on their own path keep a warp busy for its
+// longest one), the last 64 each on its own path.  What reaches beyond the run is listed (a few dozen subtrees per CTA)
+// and meets through global memory in a second kernel, with acquire/release
+// exchanges: a chain of a few microseconds per level, which inside the first kernel
+// kept whole CTAs waiting (720 us).  5.9 M leaves at D = 4: 356 + 69 us, in place of
+// the binary searches of the top-down construction (715 warp instructions per 32
+// nodes, 149 us) and of a refit that took a global acquire/release atomic and two
+// box loads per node (its barriers were half of its stalls, 660 us).
 // ---------------------------------------------------------------------------------
 
-__device__ __forceinline__ int prefix_len(const uint64_t* __restrict__ k, int n, int i, int j) {
-    if (j < 0 || j >= n) return -1;
-    const uint64_t a = k[i], b = k[j];
+constexpr int kRun = 512;        // positions per CTA
+constexpr int kRunThreads = 256;
+constexpr int kMaxDepth = 128;   // > the deepest possible tree (64 key bits + 32 position bits)
+
+__device__ __forceinline__ int key_prefix(uint64_t a, uint64_t b, int i, int j) {
     if (a == b) return 64 + __clz((unsigned)(i ^ j));
     return __clzll((long long)(a ^ b));
 }
 
-__global__ void k_karras(const uint64_t* __restrict__ k, int n, int2* __restrict__ children, int* __restrict__ parents) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
-        const int d = prefix_len(k, n, i, i + 1) - prefix_len(k, n, i, i - 1) >= 0 ? 1 : -1;
-        const int dmin = prefix_len(k, n, i, i - d);
-        int lmax = 2;
-        while (prefix_len(k, n, i, i + lmax * d) > dmin) lmax <<= 1;  // ends: past the array the length is -1
-        int l = 0;
-        for (int t = lmax >> 1; t >= 1; t >>= 1)
-            if (prefix_len(k, n, i, i + (l + t) * d) > dmin) l += t;
-        const int j = i + l * d;
-        const int dnode = prefix_len(k, n, i, j);
-        int s = 0;
-        for (int t = (l + 1) >> 1;; t = (t + 1) >> 1) {
-            if (prefix_len(k, n, i, i + (s + t) * d) > dnode) s += t;
-            if (t <= 1) break;
-        }
-        const int gamma = i + s * d + min(d, 0);
-        const int lo = min(i, j), hi = max(i, j);
-        const int left = lo == gamma ? ~gamma : gamma;
-        const int right = hi == gamma + 1 ? ~(gamma + 1) : gamma + 1;
-        children[i] = make_int2(left, right);
-        parents[left >= 0 ? left : (n - 1) + ~left] = i;
-        parents[right >= 0 ? right : (n - 1) + ~right] = i;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) parents[0] = -1;  // the root (internal node 0, or the only leaf)
-}
-
-cudaError_t karras_build(const uint64_t* sortedKeys, int n, int2* children, int* parents, cudaStream_t s) {
-    if (n <= 0) return cudaSuccess;
-    k_karras<<<blocks_for(n, 256), 256, 0, s>>>(sortedKeys, n, children, parents);
-    return cudaGetLastError();
-}
-
-constexpr int kMaxDepth = 128;  // > the deepest possible tree (64 key bits + 32 position bits)
-
-__device__ __forceinline__ unsigned atomic_add_acq_rel(unsigned* p, unsigned v) {
-    unsigned old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+__device__ __forceinline__ int exchange_acq_rel(int* p, int v) {
+    int old;
+    asm volatile("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
     return old;
 }
 
-// Bottom-up boxes: a thread starts at each leaf and climbs; at each node the
-// first of the two children to arrive stops, the second (which then finds both
-// child boxes written) computes the union and goes on.
-// READONLY: the boxes are final (point location) and go through L1; during the
-// refit another thread writes them, so they are read through L2.
+// The box of child c (c < 0: the leaf at sorted position ~c).
+// READONLY: the boxes are final (point location) and go through L1; while the tree
+// is built another thread writes them, so they are read through L2.
 template <int D, bool READONLY = false>
 __device__ __forceinline__ void child_box(const MdasDeviceGrid& g, const uint32_t* __restrict__ order, const float* boxes,
                                           int c, float (&mn)[D], float (&mx)[D]) {
@@ -616,36 +618,277 @@ __device__ __forceinline__ void child_box(const MdasDeviceGrid& g, const uint32_
 }
 
 template <int D>
-__global__ void k_refit(MdasDeviceGrid g, const uint32_t* __restrict__ order, int n, const int2* __restrict__ children,
-                        const int* __restrict__ parents, unsigned* __restrict__ visits, float* boxes) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        int node = parents[(n - 1) + p];
-        for (int depth = 0; node >= 0 && depth < kMaxDepth; ++depth) {
-            // release: the box this thread wrote last is visible to the second arrival;
-            // acquire: the second arrival sees its sibling's box
-            if (atomic_add_acq_rel(&visits[node], 1u) == 0u) break;
-            const int2 ch = children[node];
-            float amn[D], amx[D], bmn[D], bmx[D];
-            child_box<D>(g, order, boxes, ch.x, amn, amx);
-            child_box<D>(g, order, boxes, ch.y, bmn, bmx);
-            float* out = boxes + (size_t)node * 2 * D;
+struct TreeArgs {
+    MdasDeviceGrid g;
+    const uint64_t* keys;
+    const uint32_t* order;
+    int n;
+    int2* children;
+    int* parents;
+    float* boxes;
+    int* ends;  // [n - 1], -1: the far end of the first child to reach a split
+    // subtrees that climb beyond their run: ends l (bit 31: a left child) and r; their
+    // number (0 at the start)
+    uint2* pending;
+    unsigned* pendingCount;
+};
+
+// The subtree over [l, r] with its box.
+template <int D>
+struct Subtree {
+    int l, r;
+    float mn[D], mx[D];
+};
+
+// The split of the parent of [l, r]: gamma = r (left child) or l - 1; -2 for the
+// root.  key(i): the key at position i.
+template <class Key>
+__device__ __forceinline__ int parent_split(int l, int r, int n, Key key) {
+    const int dl = l > 0 ? key_prefix(key(l - 1), key(l), l - 1, l) : -1;
+    const int dr = r < n - 1 ? key_prefix(key(r), key(r + 1), r, r + 1) : -1;
+    if (dl < 0 && dr < 0) return -2;
+    return dr > dl ? r : l - 1;
+}
+
+// Joins t with its sibling across the split gamma, whose far end is `far` and whose
+// box is (smn, smx): t becomes the parent.  Returns the split of the parent's own
+// parent (-2: t is the root); id: the parent's number, cl and cr its children.
+template <int D, class Key>
+__device__ __forceinline__ int join(Subtree<D>& t, int gamma, int far, const float (&smn)[D], const float (&smx)[D],
+                                    int n, int& id, int& cl, int& cr, Key key) {
+    const bool left = t.r == gamma;  // t is the left child
+    const int l = left ? t.l : far, r = left ? far : t.r;
 #pragma unroll
-            for (int j = 0; j < D; ++j) {
-                __stcg(out + j, fminf(amn[j], bmn[j]));
-                __stcg(out + D + j, fmaxf(amx[j], bmx[j]));
+    for (int j = 0; j < D; ++j) {
+        t.mn[j] = left ? fminf(t.mn[j], smn[j]) : fminf(smn[j], t.mn[j]);
+        t.mx[j] = left ? fmaxf(t.mx[j], smx[j]) : fmaxf(smx[j], t.mx[j]);
+    }
+    t.l = l;
+    t.r = r;
+    const int up = parent_split(l, r, n, key);
+    id = up == -2 ? 0 : up == r ? r : l;
+    cl = l == gamma ? ~gamma : gamma;
+    cr = r == gamma + 1 ? ~(gamma + 1) : gamma + 1;
+    return up;
+}
+
+// Writes node id (of the split gamma) with its box.
+template <int D>
+__device__ __forceinline__ void write_node(const TreeArgs<D>& a, const Subtree<D>& t, int gamma, int id, int cl, int cr,
+                                           bool root) {
+    a.children[id] = make_int2(cl, cr);
+    a.parents[cl >= 0 ? cl : (a.n - 1) + gamma] = id;
+    a.parents[cr >= 0 ? cr : (a.n - 1) + gamma + 1] = id;
+    if (root) a.parents[0] = -1;
+    float* b = a.boxes + (size_t)id * 2 * D;
+    if constexpr (D % 2 == 0) {  // (8-byte aligned halves, 16-byte ones at D = 4)
+        if constexpr (D == 4) {
+            __stcg(reinterpret_cast<float4*>(b), make_float4(t.mn[0], t.mn[1], t.mn[2], t.mn[3]));
+            __stcg(reinterpret_cast<float4*>(b) + 1, make_float4(t.mx[0], t.mx[1], t.mx[2], t.mx[3]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < D; j += 2) {
+                __stcg(reinterpret_cast<float2*>(b + j), make_float2(t.mn[j], t.mn[j + 1]));
+                __stcg(reinterpret_cast<float2*>(b + D + j), make_float2(t.mx[j], t.mx[j + 1]));
             }
-            node = parents[node];
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            __stcg(b + j, t.mn[j]);
+            __stcg(b + D + j, t.mx[j]);
         }
     }
 }
 
-cudaError_t karras_refit(const MdasDeviceGrid& g, const uint32_t* order, int n, const int2* children,
-                         const int* parents, unsigned* visits, float* boxes, cudaStream_t s) {
-    if (n <= 1) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(visits, 0, sizeof(unsigned) * (size_t)(n - 1), s);
+// Climbs from t (whose box is in global memory) through meetings in global memory.
+template <int D>
+__device__ __forceinline__ void climb_global(const TreeArgs<D>& a, Subtree<D>& t, int gamma) {
+    auto key = [&](int i) { return a.keys[i]; };
+    for (int depth = 0; gamma != -2 && depth < kMaxDepth; ++depth) {
+        const bool left = t.r == gamma;
+        // release: the box written last is visible to the second arrival; acquire: the
+        // second arrival sees its sibling's box
+        const int far = exchange_acq_rel(&a.ends[gamma], left ? t.l : t.r);
+        if (far < 0) return;
+        const int sib = left ? (far == gamma + 1 ? ~(gamma + 1) : gamma + 1) : (far == gamma ? ~gamma : gamma);
+        float smn[D], smx[D];
+        child_box<D>(a.g, a.order, a.boxes, sib, smn, smx);
+        int id, cl, cr;
+        const int at = gamma;
+        gamma = join<D>(t, at, far, smn, smx, a.n, id, cl, cr, key);
+        write_node<D>(a, t, at, id, cl, cr, gamma == -2);
+    }
+}
+
+// A queued subtree of a run: its ends (positions in the run) and whether it is a
+// left child (then it meets its sibling at the split after its right end, else
+// before its left end).
+__device__ __forceinline__ unsigned queue_pack(int l, int r, bool left) {
+    return (unsigned)l | ((unsigned)r << 10) | ((unsigned)left << 20);
+}
+
+// Latency bounds it (a round is a chain of shared-memory steps and two barriers), so
+// what counts is how many positions an SM holds: a subtree's box takes the slot of
+// its node number, which is one of its ends (the boxes below it are not needed any
+// more), and nodes go straight to global memory.
+template <int D>
+__global__ void __launch_bounds__(kRunThreads) k_tree(TreeArgs<D> a) {
+    static_assert(kRun <= 1024, "positions in 10 bits");
+    // position p of the run at p - c0: keys (from c0 - 1), the meeting points (the
+    // split after position p; -1: nobody yet, >= 0: the first child's far end, -2:
+    // both), boxes of the subtrees that climb, by coordinate
+    __shared__ uint64_t s_keys[kRun + 2];
+    __shared__ int s_ends[kRun];
+    __shared__ unsigned s_queue[2][kRun], s_beyond[kRun];
+    __shared__ int s_count[3];  // of the queues (by round), and of s_beyond
+    __shared__ float s_box[2 * D * kRun];
+    const int c0 = blockIdx.x * kRun;
+    const int c1 = min(c0 + kRun, a.n);
+    const int t0 = threadIdx.x;
+    for (int i = t0; i < kRun + 2; i += kRunThreads) {
+        const int p = c0 - 1 + i;
+        s_keys[i] = p >= 0 && p < a.n ? a.keys[p] : 0ull;
+    }
+    auto load = [&](int i, float (&mn)[D], float (&mx)[D]) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            mn[j] = s_box[j * kRun + i];
+            mx[j] = s_box[(D + j) * kRun + i];
+        }
+    };
+    auto store = [&](int i, const float (&mn)[D], const float (&mx)[D]) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            s_box[j * kRun + i] = mn[j];
+            s_box[(D + j) * kRun + i] = mx[j];
+        }
+    };
+    for (int i = t0; i < kRun; i += kRunThreads) {
+        s_ends[i] = -1;
+        if (c0 + i < c1) {
+            float mn[D], mx[D];
+            child_box<D>(a.g, a.order, a.boxes, ~(c0 + i), mn, mx);
+            store(i, mn, mx);
+        }
+    }
+    if (t0 < 3) s_count[t0] = t0 == 0 ? c1 - c0 : 0;
+    __syncthreads();
+    auto key = [&](int i) { return s_keys[i - (c0 - 1)]; };
+    // the leaves enter the queue; then rounds until nothing climbs
+    for (int i = t0; c0 + i < c1; i += kRunThreads) {
+        const int up = parent_split(c0 + i, c0 + i, a.n, key);
+        s_queue[0][i] = queue_pack(i, i, up == c0 + i);
+    }
+    __syncthreads();
+    // One step of a subtree up its run: whether it goes on as its parent (q).
+    auto climb = [&](unsigned& q) {
+        const bool left = (q >> 20) & 1u;
+        Subtree<D> t;
+        const int li = (int)(q & 1023u), ri = (int)((q >> 10) & 1023u);
+        t.l = c0 + li;
+        t.r = c0 + ri;
+        const int gamma = left ? t.r : t.l - 1;
+        if (gamma < c0 || gamma > c1 - 2) {  // the sibling lies beyond the run
+            s_beyond[atomicAdd(&s_count[2], 1)] = q;
+            return false;
+        }
+        const int far = atomicExch(&s_ends[gamma - c0], left ? t.l : t.r);
+        if (far < 0) return false;  // first: the sibling goes on, or the sweep below
+        __threadfence_block();
+        s_ends[gamma - c0] = -2;
+        load(left ? ri : li, t.mn, t.mx);
+        float smn[D], smx[D];
+        load((left ? gamma + 1 : gamma) - c0, smn, smx);
+        int id, cl, cr;
+        const int up = join<D>(t, gamma, far, smn, smx, a.n, id, cl, cr, key);
+        store(id - c0, t.mn, t.mx);
+        write_node<D>(a, t, gamma, id, cl, cr, up == -2);
+        q = queue_pack(t.l - c0, t.r - c0, up == t.r);
+        __threadfence_block();  // the box before the next meeting
+        return up != -2;
+    };
+    int cur = 0;
+    for (; s_count[cur] > 64; cur ^= 1) {
+        const int count = s_count[cur];
+        for (int i = t0; i < count; i += kRunThreads) {
+            unsigned q = s_queue[cur][i];
+            if (climb(q)) s_queue[cur ^ 1][atomicAdd(&s_count[cur ^ 1], 1)] = q;
+        }
+        __syncthreads();
+        if (t0 == 0) s_count[cur] = 0;
+        __syncthreads();
+    }
+    // the last ones, each on its own path
+    if (t0 < s_count[cur]) {
+        unsigned q = s_queue[cur][t0];
+        for (int depth = 0; depth < kMaxDepth; ++depth)
+            if (!climb(q)) break;
+    }
+    __syncthreads();
+    // what climbs beyond the run, and the meetings that only one child reached inside
+    // it (the other comes from beyond): into the list, in one piece per run
+    for (int i = t0; i < (c1 - c0) - 1; i += kRunThreads) {
+        const int far = s_ends[i];
+        if (far < 0) continue;
+        const bool left = far <= c0 + i;
+        const int l = left ? far - c0 : i + 1, r = left ? i : far - c0;
+        s_beyond[atomicAdd(&s_count[2], 1)] = queue_pack(l, r, left);
+    }
+    __syncthreads();
+    if (t0 == 0) s_count[0] = (int)atomicAdd(a.pendingCount, (unsigned)s_count[2]);
+    __syncthreads();
+    for (int i = t0; i < s_count[2]; i += kRunThreads) {
+        const unsigned q = s_beyond[i];
+        a.pending[s_count[0] + i] = make_uint2((unsigned)(c0 + (int)(q & 1023u)) | ((q >> 20) << 31),
+                                               (unsigned)(c0 + (int)((q >> 10) & 1023u)));
+    }
+}
+
+// The subtrees that climb beyond their runs.
+template <int D>
+__global__ void __launch_bounds__(128) k_tree_top(TreeArgs<D> a) {
+    const int count = (int)*a.pendingCount;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const uint2 q = a.pending[i];
+        const bool left = q.x >> 31;
+        Subtree<D> t;
+        t.l = (int)(q.x & 0x7fffffffu);
+        t.r = (int)q.y;
+        const int gamma = left ? t.r : t.l - 1;
+        if (gamma < 0 || gamma > a.n - 2) continue;  // (the root)
+        const int id = left ? t.r : t.l;
+        child_box<D>(a.g, a.order, a.boxes, t.l == t.r ? ~id : id, t.mn, t.mx);
+        climb_global<D>(a, t, gamma);
+    }
+}
+
+template <int D>
+static cudaError_t launch_tree(const TreeArgs<D>& a, cudaStream_t s) {
+    // (as many runs per SM as its shared memory holds)
+    cudaError_t e = cudaFuncSetAttribute(k_tree<D>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
-    ORDER_SWITCH_D(g.D, (k_refit<DD><<<blocks_for(n, 256), 256, 0, s>>>(g, order, n, children, parents, visits, boxes)));
+    k_tree<D><<<(a.n + kRun - 1) / kRun, kRunThreads, 0, s>>>(a);
+    k_tree_top<D><<<8 * sm_count(), 128, 0, s>>>(a);
     return cudaGetLastError();
+}
+
+size_t tree_scratch_bytes(int n) { return 256 + sizeof(uint2) * (size_t)(n > 0 ? n : 0); }
+
+cudaError_t karras_tree(const MdasDeviceGrid& g, const uint64_t* sortedKeys, const uint32_t* order, int n,
+                        int2* children, int* parents, unsigned* visits, void* scratch, float* boxes, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    if (n == 1) return cudaMemsetAsync(parents, 0xff, sizeof(int), s);  // the only leaf has no parent
+    cudaError_t e = cudaMemsetAsync(visits, 0xff, sizeof(int) * (size_t)(n - 1), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(scratch, 0, sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    unsigned* count = static_cast<unsigned*>(scratch);
+    uint2* pending = reinterpret_cast<uint2*>(static_cast<char*>(scratch) + 256);
+    int* ends = reinterpret_cast<int*>(visits);
+    ORDER_SWITCH_D(g.D, (e = launch_tree<DD>(TreeArgs<DD>{g, sortedKeys, order, n, children, parents, boxes, ends,
+                                                          pending, count}, s)));
+    return e;
 }
 
 // Point location: depth-first, left child first, pruning with closed boxes;

@@ -41,12 +41,12 @@ int sort_launches(int n, int beginBit, int endBit);
 // children[i] = (left, right), a child c >= 0 is internal node c and c < 0 is
 // the leaf at sorted position ~c; parents[0, n-1) of internal nodes,
 // parents[n-1 + p] of the leaf at sorted position p; parent of the root = -1.
-cudaError_t karras_build(const uint64_t* sortedKeys, int n, int2* children, int* parents, cudaStream_t s);
 // Boxes of the internal nodes (2D floats each: mn, mx), unions of their
-// children's; leaf p's box is the box of grid leaf order[p].  visits: n-1
-// counters (zeroed here).
-cudaError_t karras_refit(const MdasDeviceGrid& g, const uint32_t* order, int n, const int2* children,
-                         const int* parents, unsigned* visits, float* boxes, cudaStream_t s);
+// children's; leaf p's box is the box of grid leaf order[p].  visits: n-1 words
+// of scratch; scratch: tree_scratch_bytes(n) more (at most sort_temp_bytes(n, 0, 64)).
+cudaError_t karras_tree(const MdasDeviceGrid& g, const uint64_t* sortedKeys, const uint32_t* order, int n,
+                        int2* children, int* parents, unsigned* visits, void* scratch, float* boxes, cudaStream_t s);
+size_t tree_scratch_bytes(int n);
 // For each point, the grid leaf whose box holds it (mn <= p < mx per
 // dimension, p <= mx on the domain's upper faces); the first in key order if
 // several do, -1 if none.  perm (may be null): the order in which threads take
