@@ -219,14 +219,10 @@ constexpr int kWarps = kThreads / 32;
 #ifndef MDAS_SORT_ITEMS
 #define MDAS_SORT_ITEMS 12
 #endif
-constexpr int kItems = MDAS_SORT_ITEMS;    // keys per thread
+// keys per thread (5.9 M keys, whole sort, items/CTAs per SM: 8/6 561, 8/5 526, 9/5 517,
+// 10/4 508, 12/4 500, 14/3 511, 16/3 496-500 us; 12 keeps the smaller tile for small inputs)
+constexpr int kItems = MDAS_SORT_ITEMS;
 constexpr int kTile = kThreads * kItems;  // keys per tile
-// the tile staged in digit order: static shared memory up to 12 keys per
-// thread, dynamic (keys, then values) above
-#ifndef MDAS_SORT_DYNAMIC_SMEM
-#define MDAS_SORT_DYNAMIC_SMEM (MDAS_SORT_ITEMS > 12)
-#endif
-constexpr size_t kSweepSmem = MDAS_SORT_DYNAMIC_SMEM ? (size_t)kTile * (sizeof(uint64_t) + sizeof(uint32_t)) : 0;
 constexpr unsigned kFlagAggregate = 1u << 30;
 constexpr unsigned kFlagInclusive = 2u << 30;
 constexpr unsigned kCountMask = (1u << 30) - 1u;
@@ -306,25 +302,37 @@ struct SweepArgs {
 int g_sortSpinLimit = 0;
 
 #ifndef MDAS_SORT_MIN_CTAS
-#define MDAS_SORT_MIN_CTAS 4  // 64 registers: 4 CTAs per SM (3 at 80 registers: 12 % slower)
+#define MDAS_SORT_MIN_CTAS 4  // 64 registers: 4 CTAs per SM (the sweep: see kItems)
 #endif
+// One digit position.  Cycles of a CTA's phases decide the order of the steps (5.9 M
+// keys; 608 CTAs at work at once):
+//   * ranking within the warp was the longest (16 K cycles of 38 K with eight ballots
+//     per row): a row's lanes now leave their bits at their digit in shared memory
+//     and read back the lanes that share it, the next row's bits on their way
+//     meanwhile;
+//   * the look-back (10-16 K: up to 600 predecessors that all publish at the same
+//     time, walked a window per round trip) comes after the tile is staged in digit
+//     order, which needs no global offsets: most of it is over by then (windows of 4, 8
+//     and 16 words: 488, 493, 495 us for the whole sort).
 __global__ void __launch_bounds__(kThreads, MDAS_SORT_MIN_CTAS) k_onesweep(SweepArgs a) {
     __shared__ unsigned s_warpHist[kWarps][kBins];  // per-warp digit counts, then per-warp offsets
     __shared__ unsigned s_localStart[kBins];         // digit start within the tile
     __shared__ unsigned s_globalBase[kBins];         // output position of the tile's first key of each digit
-#if MDAS_SORT_DYNAMIC_SMEM
-    extern __shared__ __align__(16) unsigned char s_tileBuf[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_tileBuf);
-    uint32_t* s_values = reinterpret_cast<uint32_t*>(s_tileBuf + sizeof(uint64_t) * kTile);
-#else
+    __shared__ unsigned s_scanWarp[kWarps];
+    // the tile staged in digit order; before that, each warp's match words (two rows of
+    // kBins, in s_keys)
     __shared__ __align__(16) uint64_t s_keys[kTile];
     __shared__ uint32_t s_values[kTile];
-#endif
+    static_assert(2 * kWarps * kBins * sizeof(unsigned) <= sizeof(s_keys), "the match words fit");
     __shared__ int s_tile;
 
     if (threadIdx.x == 0) s_tile = (int)atomicAdd(a.tileCounter, 1u);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int b = lane; b < kBins; b += 32) s_warpHist[warp][b] = 0u;
+    unsigned* match = reinterpret_cast<unsigned*>(s_keys) + warp * 2 * kBins;
+    for (int b = lane; b < kBins; b += 32) {
+        s_warpHist[warp][b] = 0u;
+        match[b] = match[kBins + b] = 0u;
+    }
     __syncthreads();
     const int tile = s_tile;
     const int tileBase = tile * kTile;
@@ -334,35 +342,42 @@ __global__ void __launch_bounds__(kThreads, MDAS_SORT_MIN_CTAS) k_onesweep(Sweep
     // load (striped per warp: item i of lane l is key warpBase + 32 i + l) and rank within the warp
     uint64_t key[kItems];
     uint32_t val[kItems];
-    unsigned digit[kItems], rank[kItems];
-    const unsigned lowerLanes = (1u << lane) - 1u;
+    unsigned rank[kItems];
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
         const int idx = warpBase + 32 * i + lane;
         const bool valid = idx < a.n;
         key[i] = valid ? a.keysIn[idx] : 0ull;
         val[i] = valid ? (a.valuesIn ? a.valuesIn[idx] : (uint32_t)idx) : 0u;
-        const unsigned d = valid ? ((unsigned)(key[i] >> a.shift) & mask) : (unsigned)kBins;  // kBins: no digit
-        digit[i] = d;
-        // lanes holding the same digit: the AND over the digit's bits of the
-        // matching ballots (cheaper than match.any, which runs on a slow pipe)
-        unsigned peers = __ballot_sync(0xffffffffu, valid);
+    }
+    auto digit = [&](uint64_t k) { return (unsigned)(k >> a.shift) & mask; };
+    auto announce = [&](int i) {  // this lane's bit at its digit, in row i's match words
+        if (warpBase + 32 * i + lane < a.n) atomicOr(&match[(i & 1) * kBins + digit(key[i])], 1u << lane);
+    };
+    const unsigned lowerLanes = (1u << lane) - 1u;
+    announce(0);
 #pragma unroll
-        for (int bit = 0; bit < 8; ++bit) {
-            const bool set = (d >> bit) & 1u;
-            const unsigned bal = __ballot_sync(0xffffffffu, set);
-            peers &= set ? bal : ~bal;
+    for (int i = 0; i < kItems; ++i) {
+        if (i + 1 < kItems) announce(i + 1);
+        __syncwarp();  // row i's bits (and the counts of row i - 1) are in place
+        const bool valid = warpBase + 32 * i + lane < a.n;
+        const unsigned d = digit(key[i]);
+        unsigned peers = 0u, base = 0u;
+        if (valid) {
+            peers = match[(i & 1) * kBins + d];
+            base = s_warpHist[warp][d];
         }
-        const int leader = __ffs(peers) - 1;
-        const unsigned base = valid ? s_warpHist[warp][d] : 0u;
-        __syncwarp();
-        if (valid && lane == leader) s_warpHist[warp][d] = base + __popc(peers);
-        __syncwarp();
+        __syncwarp();  // read by every lane
+        if (valid && (peers & lowerLanes) == 0u) {  // the digit's first lane
+            s_warpHist[warp][d] = base + __popc(peers);
+            match[(i & 1) * kBins + d] = 0u;  // for row i + 2
+        }
         rank[i] = base + __popc(peers & lowerLanes);
+        __syncwarp();
     }
     __syncthreads();
 
-    // per digit: offsets of the warps, the tile's count, publish it, look back
+    // per digit: offsets of the warps, the tile's count, published at once
     const int b = threadIdx.x;  // kThreads == kBins
     unsigned count = 0;
 #pragma unroll
@@ -373,39 +388,6 @@ __global__ void __launch_bounds__(kThreads, MDAS_SORT_MIN_CTAS) k_onesweep(Sweep
     }
     unsigned* mine = a.lookback + (size_t)tile * kBins + b;
     st_relaxed(mine, (tile == 0 ? kFlagInclusive : kFlagAggregate) | count);
-    unsigned exclusive = 0;
-    if (tile > 0) {
-        // walk back over the predecessors' words, four per round trip: add
-        // aggregates until an inclusive prefix; re-poll from a word not yet published
-        int t = tile - 1;
-        int spins = 0;
-        bool done = false;
-        while (!done && t >= 0) {
-            unsigned w[kWindow];
-#pragma unroll
-            for (int q = 0; q < kWindow; ++q)
-                w[q] = t - q >= 0 ? ld_relaxed(a.lookback + (size_t)(t - q) * kBins + b) : kFlagInclusive;
-            int q = 0;
-            for (; q < kWindow; ++q) {
-                if ((w[q] & ~kCountMask) == 0u) break;
-                exclusive += w[q] & kCountMask;
-                if (w[q] & kFlagInclusive) {
-                    done = true;
-                    break;
-                }
-            }
-            if (done) break;
-            t -= q;
-            if (q < kWindow) {  // tile t has not published yet
-                if (++spins > a.spinLimit || ld_relaxed(a.status) != 0u) {
-                    atomicOr(a.status, 1u);
-                    break;
-                }
-                __nanosleep(20);
-            }
-        }
-        st_relaxed(mine, kFlagInclusive | ((exclusive + count) & kCountMask));
-    }
 
     // digit starts within the tile (block-wide exclusive scan of the counts)
     {
@@ -415,33 +397,71 @@ __global__ void __launch_bounds__(kThreads, MDAS_SORT_MIN_CTAS) k_onesweep(Sweep
             const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += y;
         }
-        __shared__ unsigned s_scanWarp[kWarps];
         if (lane == 31) s_scanWarp[warp] = incl;
         __syncthreads();
         unsigned base = 0;
         for (int w = 0; w < warp; ++w) base += s_scanWarp[w];
-        const unsigned localStart = base + incl - count;
-        s_localStart[b] = localStart;
-        s_globalBase[b] = a.digitStart[b] + exclusive - localStart;
+        s_localStart[b] = base + incl - count;
     }
     __syncthreads();
 
-    // stage the tile in digit order, then write it out (runs of one digit are contiguous)
+    // stage the tile in digit order (the match words are not needed any more)
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
-        const unsigned d = digit[i];
-        if (d < (unsigned)kBins) {
+        if (warpBase + 32 * i + lane < a.n) {
+            const unsigned d = digit(key[i]);
             const unsigned pos = s_localStart[d] + s_warpHist[warp][d] + rank[i];
             s_keys[pos] = key[i];
             s_values[pos] = val[i];
         }
     }
+
+    // look back over the predecessors' words, a window per round trip: add aggregates
+    // until an inclusive prefix; re-poll from a word not yet published
+    unsigned exclusive = 0;
+    if (tile > 0) {
+        int t = tile - 1;
+        int spins = 0;
+        bool done = false;
+        while (!done && t >= 0) {
+            unsigned w[kWindow];
+#pragma unroll
+            for (int q = 0; q < kWindow; ++q)
+                w[q] = t - q >= 0 ? ld_relaxed(a.lookback + (size_t)(t - q) * kBins + b) : kFlagInclusive;
+            int used = 0;
+            bool open = true;
+#pragma unroll
+            for (int q = 0; q < kWindow; ++q) {
+                open = open && (w[q] & ~kCountMask) != 0u;
+                if (open) {
+                    exclusive += w[q] & kCountMask;
+                    ++used;
+                    if (w[q] & kFlagInclusive) {
+                        done = true;
+                        open = false;
+                    }
+                }
+            }
+            if (done) break;
+            t -= used;
+            if (used < kWindow) {  // tile t has not published yet
+                if (++spins > a.spinLimit || ld_relaxed(a.status) != 0u) {
+                    atomicOr(a.status, 1u);
+                    break;
+                }
+                __nanosleep(20);
+            }
+        }
+        st_relaxed(mine, kFlagInclusive | ((exclusive + count) & kCountMask));
+    }
+    s_globalBase[b] = a.digitStart[b] + exclusive - s_localStart[b];
     __syncthreads();
+
+    // write it out (runs of one digit are contiguous)
     const int tileCount = min(kTile, a.n - tileBase);
     for (int j = threadIdx.x; j < tileCount; j += kThreads) {
         const uint64_t k = s_keys[j];
-        const unsigned d = (unsigned)(k >> a.shift) & mask;
-        const unsigned dst = s_globalBase[d] + (unsigned)j;
+        const unsigned dst = s_globalBase[digit(k)] + (unsigned)j;
         if (dst < (unsigned)a.n) {  // always, unless an earlier wait gave up (then status is set)
             a.keysOut[dst] = k;
             a.valuesOut[dst] = s_values[j];
@@ -515,10 +535,6 @@ cudaError_t radix_sort(void* temp, size_t tempBytes, const uint64_t* keysIn, uin
         k_iota<<<blocks_for(n, 256), 256, 0, s>>>(valuesOut, n);
         return cudaGetLastError();
     }
-    if (kSweepSmem > 0) {
-        e = cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem);
-        if (e != cudaSuccess) return e;
-    }
     const int histBlocks = min(blocks_for(n, kThreads), 2 * sm_count());
     k_histogram<<<histBlocks, kThreads, 0, s>>>(keysIn, n, beginBit, endBit, passes, hist);
     k_digit_starts<<<passes, kBins, 0, s>>>(hist);
@@ -543,7 +559,7 @@ cudaError_t radix_sort(void* temp, size_t tempBytes, const uint64_t* keysIn, uin
         a.tileCounter = counters + p;
         a.status = status;
         a.spinLimit = g_sortSpinLimit > 0 ? g_sortSpinLimit : kSpinLimit;
-        k_onesweep<<<(unsigned)tiles, kThreads, kSweepSmem, s>>>(a);
+        k_onesweep<<<(unsigned)tiles, kThreads, 0, s>>>(a);
         srcK = a.keysOut;
         srcV = a.valuesOut;
     }
