@@ -1425,6 +1425,21 @@ __global__ void __launch_bounds__(256, 4) k_render_values(MdasDeviceGrid g, cons
 // the pixels its box covers; pixel edges advance incrementally as in the
 // reference so that the footprint is the same to the bit.
 // =====================================================================================
+// Adds to a pixel, whose line is to leave L2 last: leaves far apart in the order add to
+// the same pixels, and between them the records and sample values (64 bytes of DRAM for
+// each of the leaf's samples) stream through L2 once.  Against a plain atomicAdd:
+// 0.237 -> 0.198 ms on 4-D 1024x1024 at 16 spp, 1.50 -> 1.42 ms on 5-D 1080p at 48 spp,
+// 4.58 -> 4.51 ms on 4-D 4K at 16 spp (an image of L2's size); what runs after it does
+// not slow down.  Measured and not kept: the values marked to leave first (0.241, 1.43,
+// 4.37 ms), and the leaves of each band of rows in turn (2 bands: 0.248, 1.43, 4.40 ms).
+__device__ __forceinline__ void add_pixel(float4* p, float4 v) {
+    uint64_t policy;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
+    asm volatile("red.relaxed.gpu.global.add.L2::cache_hint.v4.f32 [%0], {%1,%2,%3,%4}, %5;" ::"l"(p), "f"(v.x),
+                 "f"(v.y), "f"(v.z), "f"(v.w), "l"(policy)
+                 : "memory");
+}
+
 // reconstruction splat of one leaf
 template <int D>
 __device__ __forceinline__ void integrate_leaf(const MdasDeviceGrid& g, const int4 node, const float (&mn)[D],
@@ -1480,7 +1495,7 @@ __device__ __forceinline__ void integrate_leaf(const MdasDeviceGrid& g, const in
                 const float4 value = make_float4((sampleValue.x * volume) * invPixArea,
                                                  (sampleValue.y * volume) * invPixArea,
                                                  (sampleValue.z * volume) * invPixArea, 0.0f);
-                atomicAdd(pixels + (size_t)y * width + x, value);
+                add_pixel(pixels + (size_t)y * width + x, value);
             }
             pMinX = pMaxX;
             pMaxX += pixelStep.x;
