@@ -228,6 +228,7 @@ constexpr unsigned kFlagInclusive = 2u << 30;
 constexpr unsigned kCountMask = (1u << 30) - 1u;
 constexpr int kSpinLimit = 1 << 18;  // polls of one look-back word before giving up
 constexpr int kMaxPasses = 8;
+constexpr int kHistKeys = 8;  // keys a thread of the histogram reads at a time
 #ifndef MDAS_SORT_WINDOW
 #define MDAS_SORT_WINDOW 4
 #endif
@@ -270,13 +271,20 @@ __global__ void __launch_bounds__(kThreads) k_histogram(const uint64_t* __restri
     __shared__ unsigned s_hist[kMaxPasses][kBins];
     for (int i = threadIdx.x; i < passes * kBins; i += kThreads) s_hist[i / kBins][i % kBins] = 0u;
     __syncthreads();
-    for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-        const uint64_t k = keys[i];
+    // kHistKeys keys of a thread at a time, so that their loads overlap (one at a time in
+    // 2 CTAs per SM, each key waited for its load: the whole sort of 5.9 M keys 473 us;
+    // 4 keys in 2, 4, 8 CTAs: 459, 455, 457; 8 keys in 4: 449)
+    const unsigned count = (unsigned)n, step = gridDim.x * kThreads;
+    for (unsigned i0 = blockIdx.x * kThreads + threadIdx.x; i0 < count; i0 += kHistKeys * step) {
+        uint64_t k[kHistKeys];
+#pragma unroll
+        for (int q = 0; q < kHistKeys; ++q) k[q] = i0 + q * step < count ? keys[i0 + q * step] : 0ull;
         for (int p = 0; p < passes; ++p) {
             const int shift = beginBit + 8 * p;
-            const int bits = min(8, endBit - shift);
-            const unsigned d = (unsigned)(k >> shift) & ((1u << bits) - 1u);
-            atomicAdd(&s_hist[p][d], 1u);
+            const unsigned m = (1u << min(8, endBit - shift)) - 1u;
+#pragma unroll
+            for (int q = 0; q < kHistKeys; ++q)
+                if (i0 + q * step < count) atomicAdd(&s_hist[p][(unsigned)(k[q] >> shift) & m], 1u);
         }
     }
     __syncthreads();
@@ -562,7 +570,7 @@ cudaError_t radix_sort(void* temp, size_t tempBytes, const uint64_t* keysIn, uin
         k_iota<<<blocks_for(n, 256), 256, 0, s>>>(valuesOut, n);
         return cudaGetLastError();
     }
-    const int histBlocks = min(blocks_for(n, kThreads), 2 * sm_count());
+    const int histBlocks = min(blocks_for(n, kThreads * kHistKeys), 4 * sm_count());
     k_histogram<<<histBlocks, kThreads, 0, s>>>(keysIn, n, beginBit, endBit, passes, hist);
     if ((e = launch_dependent(k_digit_starts, passes, kBins, s, hist)) != cudaSuccess) return e;
     const size_t tiles = ((size_t)n + kTile - 1) / kTile;
