@@ -424,7 +424,7 @@ def run_gb300(args, rank: int, world: int, local_rank: int):
                "h2d_bytes_per_step": int(prims.nbytes),
                "d2h_bytes_per_step": int(W * H * 16 + 48),  # the float4 image + the 48-byte device counters
                "ms_per_step": round(e2e_s * 1e3, 3),
-               "includes": "primitive upload, culling masks, initial sampling, every pass, integrand, "
+               "includes": "primitive upload, culling lists, initial sampling, every pass, integrand, "
                            "reconstruction, one counter read, image copy (page-locked host buffers)"}
 
     output = output_block(grid, pixels, W, H, peak)

@@ -248,8 +248,9 @@ int mdas_render(mdas_grid* g, mdas_scene* s, int budget, float* pixels, int widt
                 mdas_render_stats* stats);
 
 /* The same budget loop as one CUDA graph: the loop runs on the device (a
- * conditional while node around errors + adaptive pass + integrand for the new
- * samples + the loop condition), so a whole render costs one launch and one
+ * conditional while node around the adaptive pass, whose scan sets the loop's
+ * condition, and the values of the new samples with the errors of the split
+ * children), so a whole render costs one launch and one
  * synchronisation instead of one per pass.  Results are identical to
  * mdas_render.  The graph is built on the first call and reused while the
  * scene, budget and pixel buffer stay the same; stats->stageMs stays zero
