@@ -47,7 +47,7 @@ struct PendingTiming {
 // An instantiated device-side render (mdas_render_graph) and what it was built for.
 struct RenderGraph {
     cudaGraphExec_t exec = nullptr;
-    const void* scene = nullptr;
+    uint64_t scene = 0;  // mdas_scene::id
     int budget = 0;
     float* pixels = nullptr;
     int width = 0, height = 0;
@@ -998,7 +998,7 @@ int build_render_graph(mdas_grid* g, mdas_scene* s, int budget, float* pixels, i
         g->graph.exec = nullptr;
         return MDAS_ERR_CUDA;
     }
-    g->graph.scene = s;
+    g->graph.scene = s->id;
     g->graph.budget = budget;
     g->graph.pixels = pixels;
     g->graph.width = width;
@@ -1017,7 +1017,7 @@ int render_graph_launch(mdas_grid* g, mdas_scene* s, int budget, float* pixels, 
     if (rc) return rc;
     flush_timing(g);
     const RenderGraph& rg = g->graph;
-    if (!rg.exec || rg.scene != s || rg.budget != budget || rg.pixels != pixels || rg.width != width ||
+    if (!rg.exec || rg.scene != s->id || rg.budget != budget || rg.pixels != pixels || rg.width != width ||
         rg.height != height) {
         rc = build_render_graph(g, s, budget, pixels, width, height);
         if (rc) return rc;

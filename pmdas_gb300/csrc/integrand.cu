@@ -9,6 +9,7 @@
 #include <stdint.h>
 #include <math.h>
 #include <algorithm>
+#include <atomic>
 #include <vector>
 #include "integrand.h"
 #include "grid_types.h"
@@ -354,6 +355,15 @@ __global__ void __launch_bounds__(256) k_leaf_true_errors(MdasScene sc, const fl
         if (row < L && sub == 0) out[row] = (float)(((e + e1) + e2) * (double)volume);
     }
 }
+
+}  // namespace
+
+uint64_t mdas_next_scene_id() {
+    static std::atomic<uint64_t> last{0};
+    return ++last;
+}
+
+namespace {
 
 // splitmix64 (Steele, Lea & Flood, "Fast splittable pseudorandom number
 // generators", OOPSLA 2014): the documented stream every scene is drawn from.

@@ -37,7 +37,13 @@ int mdas_generate_scene(int kind, uint64_t seed, int count, float scaleX, float 
 // share the coordinate stride D.
 cudaError_t mdas_launch_evaluate_batch(const MdasBatchScene* scenes, int n, int D, int grid, cudaStream_t s);
 
+// A number that no other scene of the process has had (from 1; integrand.cu).
+uint64_t mdas_next_scene_id();
+
 struct mdas_scene {
+    // Tells scenes apart for what is kept between calls (the render graph of a grid):
+    // a new scene often lies at the address of a destroyed one.
+    const uint64_t id = mdas_next_scene_id();
     MdasScene desc;
     std::vector<float> prims;  // host copy
     float* d_prims = nullptr;  // device copy
