@@ -282,7 +282,8 @@ __global__ void __launch_bounds__(256) k_reference_image(MdasScene sc, const flo
 // left most of the GPU idle at the trainer's 16,384 leaves), one lane per colour
 // channel finishes it (FP64 division and square root): 16,384 leaves x 64 points of
 // a 5-D scene of 256 discs 0.93 -> 0.045 ms, the culling included.
-// cull: as k_reference_image.
+// cull: as k_reference_image; a leaf that reaches out of the scene's domain (of a grid of
+// another scale, of a loaded state) is scanned in full: the lists are for points inside.
 constexpr int kLeafLanes = 8;
 template <int D>
 __global__ void __launch_bounds__(256) k_leaf_true_errors(MdasScene sc, const float* __restrict__ prims,
@@ -310,11 +311,13 @@ __global__ void __launch_bounds__(256) k_leaf_true_errors(MdasScene sc, const fl
             const int idx[4] = {reinterpret_cast<const int*>(nb)[0], reinterpret_cast<const int*>(nb)[1],
                                 reinterpret_cast<const int*>(nb)[2], reinterpret_cast<const int*>(nb)[3]};
             float mn[D], mx[D];
+            bool inside = true;
 #pragma unroll
             for (int d = 0; d < D; ++d) {
                 mn[d] = nb[4 + d];
                 mx[d] = nb[4 + D + d];
                 volume *= mx[d] - mn[d];
+                inside = inside && mn[d] >= 0.0f && mx[d] <= (d == 0 ? sc.scaleX : d == 1 ? sc.scaleY : 1.0f);
             }
             int n = 0;
 #pragma unroll
@@ -334,8 +337,8 @@ __global__ void __launch_bounds__(256) k_leaf_true_errors(MdasScene sc, const fl
                 for (int d = 0; d < D; ++d) c[d] = mn[d] + rng.next() * (mx[d] - mn[d]);
                 skip.apply(rng);
                 float v[3];
-                if (cull) shade_culled(sc, prims, cull, c, v);
-                else mdas_shade(&sc, s_prims, c, v);
+                if (cull && inside) shade_culled(sc, prims, cull, c, v);
+                else mdas_shade(&sc, cull ? prims : s_prims, c, v);
                 acc[0] += (double)v[0];
                 acc[1] += (double)v[1];
                 acc[2] += (double)v[2];
