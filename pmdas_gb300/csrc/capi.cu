@@ -10,8 +10,10 @@
 #include <string.h>
 #include <stddef.h>
 #include <math.h>
+#include <atomic>
 #include <fstream>
 #include <string>
+#include <thread>
 #include <vector>
 #include <new>
 
@@ -1945,40 +1947,53 @@ int mdas_leaf_features(mdas_grid* g, float* features) {
 
 namespace {
 
-// Status word and loss of the standalone MLP calls, on the device and page-locked
-// on the host: 16 bytes each, one pair per host thread (of the device it last
-// called on), given back when the thread ends.  Every call waits for its stream
-// before it returns, so a thread's calls never share the words.  (Allocated and
-// freed by each call they took most of a training step: 368 us of wall time with
-// 65,536 rows, of which about 75 us ran on the GPU.)
+// Status word and loss of the standalone MLP calls.  These calls hold no object of
+// the library, so their words are module variables: nothing is allocated or freed by
+// a call (which took most of a training step: 368 us of wall time with 65,536 rows, of
+// which about 75 us ran on the GPU), every device has its own, and they come back with
+// the module after a device reset.  A call takes a slot, waits for its stream whatever
+// happened once it has queued anything, and gives the slot back; calls beyond
+// kMlpSlots at a time wait for one.
+constexpr int kMlpSlots = 64;
+__device__ unsigned mlp_words[kMlpSlots][4];
+std::atomic<uint64_t> mlpFree{~0ull};
+
 struct MlpWords {
-    int device = -1;
     unsigned* status = nullptr;  // device: status, loss
-    unsigned* host = nullptr;    // page-locked copy
     float* loss() const { return reinterpret_cast<float*>(status + 1); }
-    void release() {
-        if (status) cudaFree(status);
-        if (host) cudaFreeHost(host);
-        status = host = nullptr;
-        device = -1;
+    MlpWords() {
+        for (;;) {
+            uint64_t free = mlpFree.load(std::memory_order_relaxed);
+            if (!free) {
+                std::this_thread::yield();
+                continue;
+            }
+            bit_ = free & (~free + 1);
+            if (mlpFree.compare_exchange_weak(free, free & ~bit_, std::memory_order_acquire)) break;
+        }
     }
-    ~MlpWords() { release(); }
+    ~MlpWords() { mlpFree.fetch_or(bit_, std::memory_order_release); }
+    MlpWords(const MlpWords&) = delete;
+    MlpWords& operator=(const MlpWords&) = delete;
     bool open() {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess) return false;
-        if (dev == device) return true;
-        release();
-        if (cudaMalloc(&status, 4 * sizeof(unsigned)) != cudaSuccess ||
-            cudaMallocHost(&host, 4 * sizeof(unsigned)) != cudaSuccess) {
+        void* p = nullptr;
+        if (cudaGetSymbolAddress(&p, mlp_words) != cudaSuccess) {
             cudaGetLastError();
-            release();
             return false;
         }
-        device = dev;
+        status = static_cast<unsigned*>(p) + 4 * __builtin_ctzll(bit_);
         return true;
     }
+    // The words [0, n) into h, after everything queued on s (e: what queueing it gave).
+    cudaError_t read(unsigned* h, int n, cudaError_t e, cudaStream_t s) const {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h, status, n * sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+        const cudaError_t w = cudaStreamSynchronize(s);
+        return e != cudaSuccess ? e : w;
+    }
+
+  private:
+    uint64_t bit_ = 0;
 };
-thread_local MlpWords mlpWords;
 
 }  // namespace
 
@@ -1987,14 +2002,13 @@ extern "C" {
 int mdas_mlp_forward(const float* params, const float* features, int m, float* pred, void* stream) {
     if (!params || m < 0 || (m > 0 && (!features || !pred))) return MDAS_ERR_INVALID;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    MlpWords& w = mlpWords;
+    MlpWords w;
     if (!w.open()) return MDAS_ERR_ALLOC;
     cudaError_t e = cudaMemsetAsync(w.status, 0, sizeof(unsigned), s);
     if (e == cudaSuccess) e = mdas_mlp::forward(params, features, m, pred, w.status, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(w.host, w.status, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return MDAS_ERR_CUDA;
-    return w.host[0] ? MDAS_ERR_TIMEOUT : MDAS_OK;
+    unsigned st = 0;
+    if (w.read(&st, 1, e, s) != cudaSuccess) return MDAS_ERR_CUDA;
+    return st ? MDAS_ERR_TIMEOUT : MDAS_OK;
 }
 
 int mdas_mlp_adam(float* params, float* m1, float* m2, float* grads, int step, float learningRate, void* stream) {
@@ -2009,17 +2023,16 @@ int mdas_mlp_gradients(const float* params, const float* features, const float* 
                        float* loss, void* stream) {
     if (!params || !grads || m < 1 || !features || !targets) return MDAS_ERR_INVALID;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    MlpWords& w = mlpWords;
+    MlpWords w;
     if (!w.open()) return MDAS_ERR_ALLOC;
     cudaError_t e = cudaMemsetAsync(w.status, 0, 2 * sizeof(unsigned), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(grads, 0, sizeof(float) * MDAS_MLP_PARAMS, s);
     if (e == cudaSuccess) e = mdas_mlp::gradients(params, features, targets, m, grads, w.loss(), w.status, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(w.host, w.status, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return MDAS_ERR_CUDA;
-    if (w.host[0]) return MDAS_ERR_TIMEOUT;
+    unsigned h[2] = {0, 0};
+    if (w.read(h, 2, e, s) != cudaSuccess) return MDAS_ERR_CUDA;
+    if (h[0]) return MDAS_ERR_TIMEOUT;
     float l;
-    memcpy(&l, &w.host[1], sizeof(l));
+    memcpy(&l, &h[1], sizeof(l));
     if (loss) *loss = l / (float)m;
     return MDAS_OK;
 }
