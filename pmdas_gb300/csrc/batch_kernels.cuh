@@ -70,8 +70,11 @@ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; 
 // per pass at D = 4 on 12 images (171 M samples); with one pair per warp and
 // image, strided chunks, 61 us and the errors pass 40 -> 58 us.
 __device__ __forceinline__ int2 batch_run(int total) {
-    return make_int2((int)((long long)total * blockIdx.x / gridDim.x),
-                     (int)((long long)total * (blockIdx.x + 1) / gridDim.x));
+    // (32 bits: the two 64-bit divisions of total * CTA / CTAs took 0.8 us of every kernel,
+    // 85 passes on one 256x256 image at 16 spp 3.05 -> 2.75 ms)
+    const unsigned q = (unsigned)total / gridDim.x, r = (unsigned)total - q * gridDim.x, b = blockIdx.x;
+    const unsigned first = q * b + min(b, r);
+    return make_int2((int)first, (int)(first + q + (b < r ? 1u : 0u)));
 }
 
 // A CTA's maximum and sum added to two words (block-uniform call of 256 threads;
