@@ -2,6 +2,7 @@
 // location over the MDAS leaves (compiled with strict IEEE flags: the keys
 // depend on one division and one multiplication per coordinate, which a CPU
 // restatement must be able to repeat bit for bit).
+#include <type_traits>
 #include "order.h"
 #include "ld_hint.h"
 
@@ -645,8 +646,9 @@ __device__ __forceinline__ int exchange_acq_rel(int* p, int v) {
 }
 
 // The box of child c (c < 0: the leaf at sorted position ~c).
-// READONLY: the boxes are final (point location) and go through L1; while the tree
-// is built another thread writes them, so they are read through L2.
+// READONLY: the boxes are final (point location) and go through L1, a whole box in
+// 16-byte loads (8-byte ones at odd D, whose boxes start at multiples of 8 bytes); while
+// the tree is built another thread writes them, so they are read through L2.
 template <int D, bool READONLY = false>
 __device__ __forceinline__ void child_box(const MdasDeviceGrid& g, const uint32_t* __restrict__ order, const float* boxes,
                                           int c, float (&mn)[D], float (&mx)[D]) {
@@ -658,12 +660,32 @@ __device__ __forceinline__ void child_box(const MdasDeviceGrid& g, const uint32_
             mn[j] = h[4 + j];
             mx[j] = h[4 + D + j];
         }
+    } else if constexpr (READONLY) {
+        using V = typename std::conditional<D % 2 == 0, float4, float2>::type;
+        constexpr int W = sizeof(V) / sizeof(float);
+        const V* b = reinterpret_cast<const V*>(boxes + (size_t)c * 2 * D);
+        float v[2 * D];
+#pragma unroll
+        for (int j = 0; j < 2 * D / W; ++j) {
+            const V x = __ldg(b + j);
+            v[W * j] = x.x;
+            v[W * j + 1] = x.y;
+            if constexpr (W == 4) {
+                v[W * j + 2] = x.z;
+                v[W * j + 3] = x.w;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            mn[j] = v[j];
+            mx[j] = v[D + j];
+        }
     } else {
         const float* b = boxes + (size_t)c * 2 * D;
 #pragma unroll
         for (int j = 0; j < D; ++j) {
-            mn[j] = READONLY ? __ldg(b + j) : __ldcg(b + j);
-            mx[j] = READONLY ? __ldg(b + D + j) : __ldcg(b + D + j);
+            mn[j] = __ldcg(b + j);
+            mx[j] = __ldcg(b + D + j);
         }
     }
 }
@@ -951,8 +973,12 @@ constexpr int kStack = kMaxDepth;
 // Bound by the chain of loads down the tree (L2, about 23 levels): at a node both
 // children's boxes and both children's children are asked for together, so that a
 // level costs one round trip where a pop of one node at a time costs its box, then its
-// children, then often the other child's box.  1 M points in 5.9 M leaves: 195 -> 170 us
-// (with the boxes as 16-byte loads, which fetch what a failed first test skips: 179).
+// children, then often the other child's box.  That holds with whole boxes in wide loads
+// and every dimension tested; one 4-byte load and branch per side made a level a chain of
+// loads again and unsorted points slower than a pop at a time.  Whole calls, D = 4, pop of
+// one / both by 4-byte loads / both by wide ones: 60,000 points in 188 K leaves
+// 91 / 101 / 78 us, in 1.5 M leaves 99 / 104 / 91; 1 M points in 5.9 M leaves
+// 348 / 327 / 304; D = 6, 1 M points in 373 K leaves 356 / 396 / 346.
 // perm (may be null): the queries in the order the threads take them (points
 // sorted by a coarse Morton key, so that a warp walks one region of the tree).
 template <int D>
@@ -972,7 +998,7 @@ __global__ void k_locate(MdasDeviceGrid g, const uint32_t* __restrict__ order, i
         bool in = true;
 #pragma unroll
         for (int j = 0; j < D; ++j)
-            in = in && mn[j] <= p[j] && (p[j] < mx[j] || (p[j] == mx[j] && (c >= 0 || mx[j] >= domMx[j])));
+            in = in & (mn[j] <= p[j]) & ((p[j] < mx[j]) | ((p[j] == mx[j]) & ((c >= 0) | (mx[j] >= domMx[j]))));
         return in;
     };
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
