@@ -209,11 +209,10 @@ __device__ __forceinline__ double lanes_sum(double v) {
 // Reference image of an integrand: `spp` samples per pixel, the image plane
 // stratified on a sqrt(spp) x sqrt(spp) grid with jitter, the other dimensions
 // uniform, radiance accumulated in FP64.  T lanes share a pixel's stream and
-// its samples (the lanes of a warp then test the same few discs), so that a
-// 256 x 256 image fills the GPU too.
+// its samples (reference_lanes).
 // cull (may be null): the scene's culling lists; the samples' values are the full
 // scan's either way.
-// 4-D depth of field, 256 discs, 256 x 256 at 1024 spp: 0.89 ms; 12.8 ms with one
+// 4-D depth of field, 256 discs, 256 x 256 at 1024 spp: 0.85 ms; 12.8 ms with one
 // thread per pixel testing every disc from the front.
 template <int D, int T>
 __global__ void __launch_bounds__(256) k_reference_image(MdasScene sc, const float* __restrict__ prims,
@@ -249,7 +248,7 @@ __global__ void __launch_bounds__(256) k_reference_image(MdasScene sc, const flo
                 c[1] = ((float)y + ((float)j + rng.next()) / (float)strata) * py;
 #pragma unroll
                 for (int d = 2; d < D; ++d) c[d] = rng.next();
-                skip.apply(rng);
+                if constexpr (T > 1) skip.apply(rng);
                 float v[3];
                 if (cull) shade_culled(sc, prims, cull, c, v);
                 else mdas_shade(&sc, s_prims, c, v);
@@ -461,17 +460,48 @@ cudaError_t launch_reference_image(const MdasScene& sc, const float* d_prims, co
     }
     return cudaGetLastError();
 }
+
+// Lanes per pixel of the reference image.  A pixel's sum over its lanes costs FP64
+// additions, of which an SM makes few, so lanes are shared only
+//   * as far as that is needed to fill the GPU (2^19 of them) and each has 8 samples
+//     (us with 1, 8, 32 lanes; 4 spheres: 256x256 at 1 spp 23, 46, 128, at 64 spp 150,
+//     104, 158, at 1024 spp 2086, 1076, 1064; 3840x2160 at 1 spp 184, 2362, 12335;
+//     64x64 at 1024 spp 1934, 249, 114), on the smallest images (2^16) up to 8 whatever
+//     they have (64x64, 256 discs, at 9 spp 34, 24, 30);
+//   * up to 8 on any image where each has 256 samples: the lanes test the same few
+//     discs (640x480 at 1024 spp, 256 discs, with 1, 4, 32 lanes: 4165, 3696, 3955);
+//   * heavy: in a full scan of many primitives, which a warp leaves together only if its
+//     samples are alike, as far as few lanes are left over in the last round (640x480,
+//     64 spheres, with 1, 2, 4, 32 lanes: at 4 spp 160, 139, 142, 860, at 9 spp 333, 306,
+//     353, 875, at 64 spp 2174, 1822, 1732, 1670; 1920x1080 at 9 spp 1667, 1819, 2212,
+//     5864).
+int reference_lanes(int64_t pixels, int spp, bool heavy) {
+    int best = 1;
+    for (int t = 2; t <= 32; t *= 2) {
+        const int64_t lanes = pixels * t;
+        const bool even = (int64_t)((spp + t - 1) / t) * t * 8 <= (int64_t)spp * 9;
+        const bool few = t <= 8 && lanes <= 1 << 16 && spp >= t;
+        if (few || (heavy ? even && lanes <= (t <= 16 ? 1 << 21 : 1 << 20)
+                          : (lanes <= 1 << 19 && spp / t >= 8) || (t <= 8 && spp / t >= 256)))
+            best = t;
+    }
+    return best;
+}
 }  // namespace
 
 cudaError_t mdas_launch_reference_image(const MdasScene& sc, const float* d_prims, const unsigned* cull, int width,
                                         int height, int strata, unsigned long long seed, double* out, int sms,
                                         cudaStream_t s) {
     if (!mdas_culled_kind(sc.kind)) cull = nullptr;
-    // a warp per pixel where each lane has at least two samples, else four lanes
-    // (few samples per pixel: the sums over the lanes would cost more than the samples)
-    return strata * strata >= 64
-               ? launch_reference_image<32>(sc, d_prims, cull, width, height, strata, seed, out, sms, s)
-               : launch_reference_image<4>(sc, d_prims, cull, width, height, strata, seed, out, sms, s);
+    const bool heavy = !cull && sc.count >= 32;
+    switch (reference_lanes((int64_t)width * height, strata * strata, heavy)) {
+        case 2: return launch_reference_image<2>(sc, d_prims, cull, width, height, strata, seed, out, sms, s);
+        case 4: return launch_reference_image<4>(sc, d_prims, cull, width, height, strata, seed, out, sms, s);
+        case 8: return launch_reference_image<8>(sc, d_prims, cull, width, height, strata, seed, out, sms, s);
+        case 16: return launch_reference_image<16>(sc, d_prims, cull, width, height, strata, seed, out, sms, s);
+        case 32: return launch_reference_image<32>(sc, d_prims, cull, width, height, strata, seed, out, sms, s);
+        default: return launch_reference_image<1>(sc, d_prims, cull, width, height, strata, seed, out, sms, s);
+    }
 }
 
 // Scene generators.  Draw order is part of the format: the same seed gives the
