@@ -277,19 +277,16 @@ __global__ void __launch_bounds__(256) k_reference_image(MdasScene sc, const flo
 // over the leaf's box, estimated from `samples` uniform points with FP64
 // accumulation; err = volume * sum_c |mean_c - ref_c| / sqrt(ref_c^2 + 1e-2),
 // in the units of the plain error (a relative deviation times the volume,
-// image axes in pixels).  Eight lanes share a leaf's points (a thread per leaf
-// left most of the GPU idle at the trainer's 16,384 leaves), one lane per colour
-// channel finishes it (FP64 division and square root): 16,384 leaves x 64 points of
-// a 5-D scene of 256 discs 0.93 -> 0.045 ms, the culling included.
+// image axes in pixels).  T lanes share a leaf's points (leaf_lanes); from 4 lanes on
+// one lane per colour channel finishes it (FP64 division and square root): 16,384
+// leaves x 64 points of a 5-D scene of 256 discs 0.93 -> 0.045 ms, the culling included.
 // cull: as k_reference_image; a leaf that reaches out of the scene's domain (of a grid of
 // another scale, of a loaded state) is scanned in full: the lists are for points inside.
-constexpr int kLeafLanes = 8;
-template <int D>
+template <int D, int T>
 __global__ void __launch_bounds__(256) k_leaf_true_errors(MdasScene sc, const float* __restrict__ prims,
                                                            const unsigned* __restrict__ cull, MdasDeviceGrid g,
                                                            const int* __restrict__ leaves, int L, int samples,
                                                            unsigned long long seed, float* __restrict__ out) {
-    constexpr int T = kLeafLanes;
     extern __shared__ float s_prims[];
     if (!cull) {
         const int nfl = sc.count * MDAS_PRIM_STRIDE;
@@ -334,27 +331,42 @@ __global__ void __launch_bounds__(256) k_leaf_true_errors(MdasScene sc, const fl
                 float c[D];
 #pragma unroll
                 for (int d = 0; d < D; ++d) c[d] = mn[d] + rng.next() * (mx[d] - mn[d]);
-                skip.apply(rng);
+                if constexpr (T > 1) skip.apply(rng);
                 float v[3];
-                if (cull && inside) shade_culled(sc, prims, cull, c, v);
-                else mdas_shade(&sc, cull ? prims : s_prims, c, v);
+                // (a branch for each place of the primitives: shared-memory loads stay such)
+                if (!cull) mdas_shade(&sc, s_prims, c, v);
+                else if (inside) shade_culled(sc, prims, cull, c, v);
+                else mdas_shade(&sc, prims, c, v);
                 acc[0] += (double)v[0];
                 acc[1] += (double)v[1];
                 acc[2] += (double)v[2];
             }
         }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) acc[c] = lanes_sum<T>(acc[c]);
-        // lanes 0..2 of the leaf: one channel each
-        const double a = sub == 0 ? acc[0] : sub == 1 ? acc[1] : acc[2];
-        const float m = sub == 0 ? mean[0] : sub == 1 ? mean[1] : mean[2];
+        // the sum over the channels, on the leaf's first lane
         double e = 0.0;
-        if (row < L && sub < 3) {
-            const double ref = a / (double)samples;
-            e = fabs((double)m - ref) / sqrt(ref * ref + 1e-2);
+        if constexpr (T == 1) {
+            if (row < L) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const double ref = acc[c] / (double)samples;
+                    e += fabs((double)mean[c] - ref) / sqrt(ref * ref + 1e-2);
+                }
+            }
+        } else {
+            static_assert(T >= 4, "a lane per channel");
+#pragma unroll
+            for (int c = 0; c < 3; ++c) acc[c] = lanes_sum<T>(acc[c]);
+            // lanes 0..2 of the leaf: one channel each
+            const double a = sub == 0 ? acc[0] : sub == 1 ? acc[1] : acc[2];
+            const float m = sub == 0 ? mean[0] : sub == 1 ? mean[1] : mean[2];
+            if (row < L && sub < 3) {
+                const double ref = a / (double)samples;
+                e = fabs((double)m - ref) / sqrt(ref * ref + 1e-2);
+            }
+            const double e1 = __shfl_down_sync(0xffffffffu, e, 1), e2 = __shfl_down_sync(0xffffffffu, e, 2);
+            e = (e + e1) + e2;
         }
-        const double e1 = __shfl_down_sync(0xffffffffu, e, 1), e2 = __shfl_down_sync(0xffffffffu, e, 2);
-        if (row < L && sub == 0) out[row] = (float)(((e + e1) + e2) * (double)volume);
+        if (row < L && sub == 0) out[row] = (float)(e * (double)volume);
     }
 }
 
@@ -384,23 +396,53 @@ struct SplitMix64 {
 
 }  // namespace
 
+namespace {
+template <int T>
+cudaError_t launch_leaf_true_errors(const MdasScene& sc, const float* d_prims, const unsigned* cull,
+                                    const MdasDeviceGrid& g, const int* leaves, int L, int samples,
+                                    unsigned long long seed, float* out, cudaStream_t s) {
+    const size_t smem = cull ? 0 : sizeof(float) * MDAS_PRIM_STRIDE * (size_t)sc.count;
+    const int perBlock = 256 / T;
+    const int64_t want = ((int64_t)L + perBlock - 1) / perBlock;
+    const int grid = (int)(want < 65535 ? want : 65535);
+    switch (g.D) {
+        case 3: k_leaf_true_errors<3, T><<<grid, 256, smem, s>>>(sc, d_prims, cull, g, leaves, L, samples, seed, out); break;
+        case 4: k_leaf_true_errors<4, T><<<grid, 256, smem, s>>>(sc, d_prims, cull, g, leaves, L, samples, seed, out); break;
+        case 5: k_leaf_true_errors<5, T><<<grid, 256, smem, s>>>(sc, d_prims, cull, g, leaves, L, samples, seed, out); break;
+        case 6: k_leaf_true_errors<6, T><<<grid, 256, smem, s>>>(sc, d_prims, cull, g, leaves, L, samples, seed, out); break;
+        default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+// Lanes per leaf of the true errors: 1, 4 or 8.  Lanes are shared
+//   * as far as that is needed to fill the GPU and each has 4 samples (us with 1, 4, 8
+//     lanes, 256 discs: 20,000 leaves with 16 points 66, 53, 58, with 64 points 132, 72,
+//     72; 665,000 leaves with 1 point 212, 333, 643, with 64 points 804, 799, 1037; 4
+//     spheres, 100,000 leaves with 16 points 107, 102, 130), 4 on the fewest leaves
+//     whatever they have (5000 with 1 point 44, 38, 46);
+//   * heavy: as reference_lanes (256 spheres, 629,000 leaves: with 1 point 503, 1400,
+//     2472, with 4 points 1749, 1416, 2492, with 16 points 6721, 5264, 4784).
+int leaf_lanes(int L, int samples, bool heavy) {
+    int best = 4LL * L <= 1 << 15 ? 4 : 1;
+    for (int t = 4; t <= 8; t *= 2) {
+        const bool even = ((int64_t)samples + t - 1) / t * t * 8 <= (int64_t)samples * 9;
+        if (heavy ? even : (int64_t)L * t <= 1 << 19 && samples / t >= 4) best = t;
+    }
+    return best;
+}
+}  // namespace
+
 cudaError_t mdas_launch_leaf_true_errors(const MdasScene& sc, const float* d_prims, const unsigned* cull,
                                          const MdasDeviceGrid& g, const int* leaves, int L, int samples,
                                          unsigned long long seed, float* out, cudaStream_t s) {
     if (L <= 0) return cudaSuccess;
     if (!mdas_culled_kind(sc.kind)) cull = nullptr;
-    const size_t smem = cull ? 0 : sizeof(float) * MDAS_PRIM_STRIDE * (size_t)sc.count;
-    const int perBlock = 256 / kLeafLanes;
-    const int64_t want = ((int64_t)L + perBlock - 1) / perBlock;
-    const int grid = (int)(want < 65535 ? want : 65535);
-    switch (g.D) {
-        case 3: k_leaf_true_errors<3><<<grid, 256, smem, s>>>(sc, d_prims, cull, g, leaves, L, samples, seed, out); break;
-        case 4: k_leaf_true_errors<4><<<grid, 256, smem, s>>>(sc, d_prims, cull, g, leaves, L, samples, seed, out); break;
-        case 5: k_leaf_true_errors<5><<<grid, 256, smem, s>>>(sc, d_prims, cull, g, leaves, L, samples, seed, out); break;
-        case 6: k_leaf_true_errors<6><<<grid, 256, smem, s>>>(sc, d_prims, cull, g, leaves, L, samples, seed, out); break;
-        default: return cudaErrorInvalidValue;
+    switch (leaf_lanes(L, samples, !cull && sc.count >= 32)) {
+        case 4: return launch_leaf_true_errors<4>(sc, d_prims, cull, g, leaves, L, samples, seed, out, s);
+        case 8: return launch_leaf_true_errors<8>(sc, d_prims, cull, g, leaves, L, samples, seed, out, s);
+        default: return launch_leaf_true_errors<1>(sc, d_prims, cull, g, leaves, L, samples, seed, out, s);
     }
-    return cudaGetLastError();
 }
 
 size_t mdas_cull_words(const MdasScene& sc) {
@@ -479,7 +521,7 @@ int reference_lanes(int64_t pixels, int spp, bool heavy) {
     int best = 1;
     for (int t = 2; t <= 32; t *= 2) {
         const int64_t lanes = pixels * t;
-        const bool even = (int64_t)((spp + t - 1) / t) * t * 8 <= (int64_t)spp * 9;
+        const bool even = ((int64_t)spp + t - 1) / t * t * 8 <= (int64_t)spp * 9;
         const bool few = t <= 8 && lanes <= 1 << 16 && spp >= t;
         if (few || (heavy ? even && lanes <= (t <= 16 ? 1 << 21 : 1 << 20)
                           : (lanes <= 1 << 19 && spp / t >= 8) || (t <= 8 && spp / t >= 256)))
