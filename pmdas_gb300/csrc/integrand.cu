@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256) k_leaf_true_errors(MdasScene sc, const fl
             for (int c = 0; c < 3; ++c) mean[c] = n ? mean[c] / (float)n : 0.0f;
             Lcg64 rng{seed ^ (0x9E3779B97F4A7C15ull * (unsigned long long)(i + 1))};
             start.apply(rng);
-            for (int s = sub; s < samples; s += T) {
+            for (unsigned s = sub; s < (unsigned)samples; s += T) {  // (past 2^31 - 1 near its end)
                 float c[D];
 #pragma unroll
                 for (int d = 0; d < D; ++d) c[d] = mn[d] + rng.next() * (mx[d] - mn[d]);
