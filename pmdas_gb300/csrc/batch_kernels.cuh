@@ -292,8 +292,12 @@ __global__ void __launch_bounds__(256) k_batch_initial_errors(const MdasBatchIma
 }
 
 // ---- the pass's new samples: values, and errors of the split children
-// (k_render_values over the images)
-template <int D>
+// (k_render_values over the images).  FULL: of the images without culling lists, else of
+// the others: an instance for both spilled 84 bytes and was slower than an integrand
+// kernel and an errors kernel for direct light (two images of 4-D 256x256 and two of
+// 512x512 with 4 spheres: 2.43 ms with two kernels, 2.50 with one instance for both, 2.40
+// with this).
+template <int D, bool FULL>
 __global__ void __launch_bounds__(256, 4) k_batch_values(const MdasBatchImage* __restrict__ imgs,
                                                       const MdasBatchScene* __restrict__ scenes, int n) {
     __shared__ int s_pre[MDAS_MAX_BATCH + 1];
@@ -302,7 +306,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_values(const MdasBatchImage* _
     // (an image without an accepted leaf gets a chunk too: one CTA sets its g_error)
     const int total = batch_prefix(n, s_pre, s_warp, [&](int i) {
         const MdasDeviceGrid& g = imgs[i].g;
-        return g.counts->active ? max(ceil_div(g.counts->newN, 256), 1) : 0;
+        return g.counts->active && (scenes[i].cull == nullptr) == FULL ? max(ceil_div(g.counts->newN, 256), 1) : 0;
     });
     int cur = -1;  // the image of the running maximum (uniform across the block)
     float maxError = 0.0f;
@@ -321,8 +325,8 @@ __global__ void __launch_bounds__(256, 4) k_batch_values(const MdasBatchImage* _
         }
         const bool more = g.ctl->more != 0;
         const MdasBatchScene& b = scenes[i];
-        const float m = render_sample<D>(g, b.sc, b.prims, b.cull, (ch - s_pre[i]) * 256 + threadIdx.x, g.counts->newN,
-                                         g.ctl->N0, g.ctl->L0, more);
+        const float m = render_sample<D, FULL>(g, b.sc, b.prims, b.cull, (ch - s_pre[i]) * 256 + threadIdx.x,
+                                               g.counts->newN, g.ctl->N0, g.ctl->L0, more);
         maxError = fmaxf(maxError, m);
         if (more && ch == s_pre[i] && threadIdx.x == 0) {  // the image's first chunk
             maxError = fmaxf(maxError, __uint_as_float(g.counts->gerrCarry));
@@ -529,10 +533,14 @@ cudaError_t batch_initial_errors(const MdasBatchImage* imgs, int n, int D, int g
     return cudaGetLastError();
 }
 
-cudaError_t batch_values(const MdasBatchImage* imgs, const MdasBatchScene* scenes, int n, int D, int grid,
-                         cudaStream_t s) {
+// culled, full: whether any image has, or has no, culling lists.
+cudaError_t batch_values(const MdasBatchImage* imgs, const MdasBatchScene* scenes, int n, int D, bool culled,
+                         bool full, int grid, cudaStream_t s) {
     cudaError_t e = cudaSuccess;
-    MDAS_BATCH_SWITCH_D(D, (e = launch_pdl(k_batch_values<DD>, grid, 256, s, imgs, scenes, n)));
+    if (culled) MDAS_BATCH_SWITCH_D(D, (e = launch_pdl(k_batch_values<DD, false>, grid, 256, s, imgs, scenes, n)));
+    // (a launch behind the other instance's waits for it whole: that one waited for place)
+    if (e == cudaSuccess && full)
+        MDAS_BATCH_SWITCH_D(D, (e = launch_on(k_batch_values<DD, true>, !culled, grid, 256, 0, s, imgs, scenes, n)));
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 

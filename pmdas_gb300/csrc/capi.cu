@@ -1067,6 +1067,7 @@ struct mdas_batch {
     std::vector<int> order;          // batch slot -> caller index (images grouped by dimension)
     struct Group {
         int D, offset, count;
+        bool culled, full;  // whether any of its scenes has, or has no, culling lists
     };
     std::vector<Group> groups;
     std::vector<MdasBatchImage> himgs;
@@ -1136,7 +1137,8 @@ cudaError_t enqueue_batch_body(mdas_batch* b, cudaGraphConditionalHandle handle,
         if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_scan, imgs, gr.count, kMaxGraphPasses, gs);
         if (e == cudaSuccess) e = MDAS_ARITH_CALL(b, batch_place, imgs, gr.count, gr.D, gPl, gs);
         if (e == cudaSuccess)
-            e = MDAS_ARITH_CALL(b, batch_values, imgs, b->d_scenes + gr.offset, gr.count, gr.D, gVal, gs);
+            e = MDAS_ARITH_CALL(b, batch_values, imgs, b->d_scenes + gr.offset, gr.count, gr.D, gr.culled, gr.full, gVal,
+                                gs);
         if (k > 0 && e == cudaSuccess) e = cudaEventRecord(b->joinEvent[k], gs);
     }
     for (size_t k = 1; k < b->groups.size() && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(s, b->joinEvent[k], 0);
@@ -1249,7 +1251,7 @@ int mdas_batch_create(mdas_batch** out, int n, mdas_grid* const* grids, mdas_sce
         const int off = (int)b->order.size();
         for (int i = 0; i < n; ++i)
             if (grids[i]->dg.D == D) b->order.push_back(i);
-        if ((int)b->order.size() > off) b->groups.push_back({D, off, (int)b->order.size() - off});
+        if ((int)b->order.size() > off) b->groups.push_back({D, off, (int)b->order.size() - off, false, false});
     }
     for (int slot = 0; slot < n; ++slot) {
         const int i = b->order[slot];
@@ -1289,6 +1291,8 @@ int mdas_batch_create(mdas_batch** out, int n, mdas_grid* const* grids, mdas_sce
         bs.dim = g->dg.D;
         bs.initialSamples = (int)(4 * L0);
         b->hscenes.push_back(bs);
+        for (auto& gr : b->groups)
+            if (gr.D == g->dg.D) (bs.cull ? gr.culled : gr.full) = true;
     }
     bool ok = cudaMalloc(&b->d_imgs, sizeof(MdasBatchImage) * n) == cudaSuccess &&
               cudaMalloc(&b->d_scenes, sizeof(MdasBatchScene) * n) == cudaSuccess &&

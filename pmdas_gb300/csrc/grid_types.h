@@ -173,7 +173,7 @@ struct MdasBatchScene {
     cudaError_t batch_set_counts(const MdasBatchImage* imgs, int n, cudaStream_t s);                         \
     cudaError_t batch_initial_errors(const MdasBatchImage* imgs, int n, int D, int grid, cudaStream_t s);    \
     cudaError_t batch_values(const MdasBatchImage* imgs, const MdasBatchScene* scenes, int n, int D,         \
-                             int grid, cudaStream_t s);                                                      \
+                             bool culled, bool full, int grid, cudaStream_t s);                              \
     cudaError_t batch_reset(const MdasBatchImage* imgs, int n, int which, cudaStream_t s);                   \
     cudaError_t batch_decide(const MdasBatchImage* imgs, int n, int D, int K, bool learned, int grid,        \
                              cudaStream_t s);                                                                 \

@@ -30,6 +30,7 @@ extern "C" {
 // depth-of-field scenes list their discs by increasing depth (stable order).
 // Spheres: [cx, cy, cz, r, 0, 0, 1/r, r*r, 0, 0, 0, 0].
 #define MDAS_PRIM_STRIDE 12
+#define MDAS_MAX_PRIMS 1024  // 48 KB of shared memory in the kernels that test every primitive
 
 typedef struct MdasScene {
     int kind;

@@ -1350,10 +1350,14 @@ __global__ void __launch_bounds__(256, D >= 5 ? 2 : 3) k_adaptive_place(MdasDevi
 // =====================================================================================
 // The sample of rank k (its group's warp calls this together; k >= accepted: a lane
 // without one).  Returns the larger error of its children (0 without).
-template <int D>
-__device__ __forceinline__ float render_sample(const MdasDeviceGrid& g, const MdasScene& sc,
-                                               const float* __restrict__ prims, const unsigned* __restrict__ cull, int k,
-                                               int accepted, int N, int L, bool more) {
+// The old values gathered here all lie below N, the values written at N and above, so
+// the read-only loads (ld_value64) never touch a word that this kernel writes.
+// FULL: a scene without culling lists.  Its scan of all primitives is long and needs the
+// registers, so the gathers follow it; a culled sample's few tests run under the gathers.
+template <int D, bool FULL>
+__device__ __forceinline__ float render_sample(const MdasDeviceGrid& g, const MdasScene& sc, const float* prims,
+                                               const unsigned* __restrict__ cull, int k, int accepted, int N, int L,
+                                               bool more) {
     const bool active = k < accepted;
     const size_t s = (size_t)N + k;
     float c[D];
@@ -1364,6 +1368,10 @@ __device__ __forceinline__ float render_sample(const MdasDeviceGrid& g, const Md
         for (int d = 0; d < D; ++d) c[d] = g.coords[s * D + d];
     }
     const bool split = active && more && rank >= 0;
+    float val[3] = {0.0f, 0.0f, 0.0f};
+    if constexpr (FULL) {
+        if (active) mdas_shade(&sc, prims, c, val);
+    }
     int4 l = make_int4(0, 0, 0, 0), r = l;
     float3 v[5];
     if (split) {
@@ -1374,10 +1382,8 @@ __device__ __forceinline__ float render_sample(const MdasDeviceGrid& g, const Md
         for (int i = 0; i < 5; ++i)
             if (idx[i] != N + k) v[i] = ld_value64(g.values, idx[i]);
     }
-    float val[3] = {0.0f, 0.0f, 0.0f};
-    if (active) {
-        if (cull) shade_culled(sc, prims, cull, c, val);
-        else mdas_shade(&sc, prims, c, val);
+    if constexpr (!FULL) {
+        if (active) shade_culled(sc, prims, cull, c, val);
     }
     __syncwarp();  // the group's notes are read: its values may take their place
     if (active) {
@@ -1404,17 +1410,28 @@ __device__ __forceinline__ float render_sample(const MdasDeviceGrid& g, const Md
     return fmaxf(errL, errR);
 }
 
-template <int D>
+// FULL: the primitives are staged in (dynamic) shared memory.  4-D direct light,
+// 1280x720 at 4 spp, with the integrand in a kernel of its own / one variant for both
+// kinds of scene, primitives in global memory / this: 4 spheres 1.05 / 0.98 / 0.98 ms,
+// 128 spheres 3.31 / 3.65 / 3.22, 1024 spheres 16.8 / 22.0 / 16.8.
+template <int D, bool FULL>
 __global__ void __launch_bounds__(256, 4) k_render_values(MdasDeviceGrid g, const __grid_constant__ MdasScene sc,
                                                        const float* __restrict__ prims,
                                                        const unsigned* __restrict__ cull) {
     __shared__ unsigned s_max[8];
+    extern __shared__ float s_prims[];
+    if constexpr (FULL) {
+        const int nfl = sc.count * MDAS_PRIM_STRIDE;
+        for (int k = threadIdx.x; k < nfl; k += 256) s_prims[k] = prims[k];
+        __syncthreads();
+    }
     pdl_wait();
     const int N = g.ctl->N0, L = g.ctl->L0, accepted = g.counts->newN;
     const bool more = g.ctl->more != 0;
     float maxError = 0.0f;
     for (int base = blockIdx.x * 256; base < accepted; base += gridDim.x * 256)
-        maxError = fmaxf(maxError, render_sample<D>(g, sc, prims, cull, base + threadIdx.x, accepted, N, L, more));
+        maxError = fmaxf(maxError, render_sample<D, FULL>(g, sc, FULL ? s_prims : prims, cull, base + threadIdx.x,
+                                                          accepted, N, L, more));
     if (!more) return;
     // g_error for the next pass: over the children and the leaves the pass kept
     // (kdgrid.cu:684-716 takes it over all leaves)
@@ -1729,11 +1746,12 @@ __global__ void __launch_bounds__(256) k_learned_judge(MdasDeviceGrid g, int Lho
 // A launch that may overlap the tail of the previous kernel on the stream (the
 // kernel calls pdl_wait() before it reads what that kernel wrote).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_on(void (*kernel)(KArgs...), bool dependent, int grid, int block, cudaStream_t s, Args... args) {
+cudaError_t launch_on(void (*kernel)(KArgs...), bool dependent, int grid, int block, size_t smem, cudaStream_t s,
+                      Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1745,7 +1763,7 @@ cudaError_t launch_on(void (*kernel)(KArgs...), bool dependent, int grid, int bl
 
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args... args) {
-    return launch_on(kernel, true, grid, block, s, args...);
+    return launch_on(kernel, true, grid, block, 0, s, args...);
 }
 
 #define MDAS_SWITCH_D(D, EXPR)                 \
@@ -1807,13 +1825,13 @@ static cudaError_t launch_decide(const MdasDeviceGrid& g, bool dependent, int gr
     unsigned A, C;
     lcg_jump((unsigned)(g.candidatesNum * g.D), &A, &C);
     if (g.priority && g.tileK == 4) {
-        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 4, true>, dependent, grid, 256, s, g, A, C)));
+        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 4, true>, dependent, grid, 256, 0, s, g, A, C)));
     } else if (g.priority) {
-        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 8, true>, dependent, grid, 256, s, g, A, C)));
+        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 8, true>, dependent, grid, 256, 0, s, g, A, C)));
     } else if (g.tileK == 4) {
-        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 4, false>, dependent, grid, 256, s, g, A, C)));
+        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 4, false>, dependent, grid, 256, 0, s, g, A, C)));
     } else {
-        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 8, false>, dependent, grid, 256, s, g, A, C)));
+        MDAS_SWITCH_D(g.D, (e = launch_on(k_adaptive_decide<DD, 8, false>, dependent, grid, 256, 0, s, g, A, C)));
     }
     return e;
 }
@@ -1842,8 +1860,21 @@ cudaError_t render_pass(const MdasDeviceGrid& g, const MdasScene& sc, const floa
     cudaError_t e = launch_decide(g, g.priority != nullptr, gridDecide, s);
     if (e == cudaSuccess) e = launch_pdl(k_loop_scan, 1, 1024, s, g, h, budget, maxPasses);
     if (e == cudaSuccess) e = launch_place(g, true, gridPlace, s);
-    if (e == cudaSuccess)
-        MDAS_SWITCH_D(g.D, (e = launch_pdl(k_render_values<DD>, gridValues, 256, s, g, sc, prims, cull)));
+    if (e == cudaSuccess && cull) {
+        MDAS_SWITCH_D(g.D, (e = launch_pdl(k_render_values<DD, false>, gridValues, 256, s, g, sc, prims, cull)));
+    } else if (e == cudaSuccess) {
+        const size_t smem = sizeof(float) * MDAS_PRIM_STRIDE * (size_t)sc.count;
+        // a sample of many primitives takes long: CTAs beyond the resident ones even out
+        // the last wave (1920x1080 at 8 spp, 128 spheres 8.41 -> 8.15 ms; 4 spheres 2.77
+        // -> 2.80)
+        const int grid = sc.count >= 128 ? 4 * gridValues : gridValues;
+        // (the same limit from every thread and for every scene)
+        constexpr int kMost = (int)sizeof(float) * MDAS_PRIM_STRIDE * MDAS_MAX_PRIMS;
+        MDAS_SWITCH_D(g.D, (e = cudaFuncSetAttribute(k_render_values<DD, true>,
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kMost)));
+        if (e != cudaSuccess) return e;
+        MDAS_SWITCH_D(g.D, (e = launch_on(k_render_values<DD, true>, true, grid, 256, smem, s, g, sc, prims, cull)));
+    }
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
@@ -1919,7 +1950,7 @@ int max_blocks_per_sm(int D, int which) {
             MDAS_SWITCH_D(D, (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_integrate<DD>, 256, 0)));
             break;
         case MDAS_K_RENDER_VALUES:
-            MDAS_SWITCH_D(D, (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_render_values<DD>, 256, 0)));
+            MDAS_SWITCH_D(D, (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_render_values<DD, false>, 256, 0)));
             break;
         case MDAS_K_DECIDE:
             MDAS_SWITCH_D(D, (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adaptive_decide<DD, 8, false>,

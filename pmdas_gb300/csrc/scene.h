@@ -7,8 +7,6 @@
 #include "integrand.h"
 #include "grid_types.h"
 
-#define MDAS_MAX_PRIMS 1024  // 48 KB of shared memory in the integrand kernel
-
 // The culling lists of a scene (shade.cuh).
 size_t mdas_cull_words(const MdasScene& sc);  // 0: the scene kind is not culled
 cudaError_t mdas_launch_build_cull(const MdasScene& sc, const float* d_prims, unsigned* lists, cudaStream_t s);
