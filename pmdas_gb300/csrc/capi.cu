@@ -936,32 +936,35 @@ int build_render_graph(mdas_grid* g, mdas_scene* s, int budget, float* pixels, i
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
     if (e != cudaSuccess) return MDAS_ERR_CUDA;
-    auto fail = [&](cudaError_t err) {
+    bool bodyLost = false;
+    auto fail = [&]() {
         cudaGraph_t junk = nullptr;
         cudaStreamEndCapture(cs, &junk);
-        if (junk) cudaGraphDestroy(junk);
+        // (a failed launch in the loop's body ends its capture and takes the body graph
+        // with it; destroying the graph around it then crashes, so it is left)
+        if (junk && !bodyLost) cudaGraphDestroy(junk);
         cudaGetLastError();
-        return err == cudaSuccess ? MDAS_ERR_CUDA : MDAS_ERR_CUDA;
+        return MDAS_ERR_CUDA;
     };
     // prologue: initial sampling + integrand for all initial samples
     e = g->arith == MDAS_ARITH_IEEE ? mdas_ieee::initial_sampling(d, (int)L0, cs)
                                     : mdas_fast::initial_sampling(d, (int)L0, cs);
-    if (e != cudaSuccess) return fail(e);
+    if (e != cudaSuccess) return fail();
     k_set_counts<<<1, 1, 0, cs>>>(d.counts, (int)N0, (int)L0);
     e = mdas_launch_evaluate(s->desc, s->d_prims, s->d_cull, d.coords, d.values, d.D, nullptr, 0, (int)N0, gEval, cs);
     // (a render without a pass leaves the errors uncomputed, as the host loop does)
     if (e == cudaSuccess && firstPass) e = MDAS_GRID_CALL(g, compute_errors, d, gErr, false, cs);
-    if (e != cudaSuccess) return fail(e);
+    if (e != cudaSuccess) return fail();
     // the conditional while node
     cudaStreamCaptureStatus status;
     cudaGraph_t capGraph = nullptr;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
     e = cudaStreamGetCaptureInfo(cs, &status, nullptr, &capGraph, &deps, nullptr, &ndeps);
-    if (e != cudaSuccess) return fail(e);
+    if (e != cudaSuccess) return fail();
     cudaGraphConditionalHandle handle;
     e = cudaGraphConditionalHandleCreate(&handle, capGraph, firstPass, cudaGraphCondAssignDefault);
-    if (e != cudaSuccess) return fail(e);
+    if (e != cudaSuccess) return fail();
     cudaGraphNodeParams cp = {};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = handle;
@@ -969,13 +972,13 @@ int build_render_graph(mdas_grid* g, mdas_scene* s, int budget, float* pixels, i
     cp.conditional.size = 1;
     cudaGraphNode_t condNode;
     e = cudaGraphAddNode(&condNode, capGraph, deps, nullptr, ndeps, &cp);
-    if (e != cudaSuccess) return fail(e);
+    if (e != cudaSuccess) return fail();
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     e = cudaStreamUpdateCaptureDependencies(cs, &condNode, nullptr, 1, cudaStreamSetCaptureDependencies);
-    if (e != cudaSuccess) return fail(e);
+    if (e != cudaSuccess) return fail();
     // loop body, captured into the conditional node's child graph
     e = cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-    if (e != cudaSuccess) return fail(e);
+    if (e != cudaSuccess) return fail();
     cudaError_t eb = cudaSuccess;
     if (g->learned) {
         eb = learned_queue(g, -1, bs);  // predictions and the judge's verdict for this pass
@@ -987,11 +990,12 @@ int build_render_graph(mdas_grid* g, mdas_scene* s, int budget, float* pixels, i
     g->dg.priority = nullptr;
     cudaGraph_t bodyOut = nullptr;
     e = cudaStreamEndCapture(bs, &bodyOut);
-    if (eb != cudaSuccess || e != cudaSuccess) return fail(eb != cudaSuccess ? eb : e);
+    bodyLost = e != cudaSuccess;
+    if (eb != cudaSuccess || e != cudaSuccess) return fail();
     // epilogue: reconstruction
     e = g->arith == MDAS_ARITH_IEEE ? mdas_ieee::integrate(d, gInt, pixels, width, height, cs)
                                     : mdas_fast::integrate(d, gInt, pixels, width, height, cs);
-    if (e != cudaSuccess) return fail(e);
+    if (e != cudaSuccess) return fail();
     e = cudaStreamEndCapture(cs, &graph);
     if (e != cudaSuccess) return MDAS_ERR_CUDA;
     e = cudaGraphInstantiate(&g->graph.exec, graph, 0);
@@ -1164,10 +1168,11 @@ int build_batch_graph(mdas_batch* b) {
     cudaStream_t cs = b->captureStream, bs = b->bodyStream;
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
     if (e != cudaSuccess) return MDAS_ERR_CUDA;
+    bool bodyLost = false;  // (as build_render_graph)
     auto fail = [&]() {
         cudaGraph_t junk = nullptr;
         cudaStreamEndCapture(cs, &junk);
-        if (junk) cudaGraphDestroy(junk);
+        if (junk && !bodyLost) cudaGraphDestroy(junk);
         cudaGetLastError();
         return MDAS_ERR_CUDA;
     };
@@ -1196,6 +1201,7 @@ int build_batch_graph(mdas_batch* b) {
     const cudaError_t eb = enqueue_batch_body(b, handle, nullptr, bs);
     cudaGraph_t bodyOut = nullptr;
     e = cudaStreamEndCapture(bs, &bodyOut);
+    bodyLost = e != cudaSuccess;
     if (eb != cudaSuccess || e != cudaSuccess) return fail();
     if (enqueue_batch_epilogue(b, cs) != cudaSuccess) return fail();
     cudaGraph_t graph = nullptr;
