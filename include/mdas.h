@@ -283,8 +283,10 @@ int mdas_batch_render(mdas_batch* b, mdas_render_stats* stats);
  * verdict per pass) instead of the graph's device-side loop.  Same results;
  * for tools that cannot look inside a graph's conditional node (profilers). */
 int mdas_batch_render_stepped(mdas_batch* b, mdas_render_stats* stats);
-/* Persistent CTAs per SM of the errors, decide, place and integrate/integrand
- * launches (rebuilds the graph). */
+/* CTAs per SM (rebuilds the graph) of, in this order: the errors of the initial
+ * leaves, decide, place, and the launches over samples and pixels (initial
+ * sampling, integrand, each pass's values with the errors of its split
+ * children, reconstruction). */
 int mdas_batch_set_tuning(mdas_batch* b, const int* ctasPerSm4);
 /* mdas_batch_set_tuning plus the tile size of the adaptive pass's decide
  * kernel (leavesPerTile: 1024 or 2048 leaves per 256-thread tile).  The

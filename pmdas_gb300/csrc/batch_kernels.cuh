@@ -1,11 +1,12 @@
 // batch_kernels.cuh — many images of uneven size, dimension and budget in one
 // launch per stage (compiled inside MDAS_NS after kdgrid_kernels.cuh).
 //
-// Each stage enumerates its work items (initial cells, error leaves, tiles of
-// 1024 leaves, accepted leaves, reconstruction leaves) across all images of the
-// launch: every CTA computes the per-image item counts from the images' device
-// counters and their prefix in shared memory, then walks the global item range
-// with a grid stride, mapping each chunk of items to its image by binary search.
+// Each stage enumerates its work items (initial cells, leaves, decide tiles of 1024
+// or 2048 leaves, accepted leaves, new samples) across all images of the launch:
+// every CTA computes the per-image item counts from the images' device counters and
+// their prefix in shared memory, then walks the global item range with a grid stride
+// or takes one run of it (batch_run), mapping each chunk of items to its image by
+// binary search.
 // A chunk never spans two images, so every block-wide step (scan, reduction)
 // stays within one image.  Per image the work and its results are exactly those
 // of the single-image kernels: the item bodies are the same device functions.
@@ -296,7 +297,9 @@ __global__ void __launch_bounds__(256) k_batch_initial_errors(const MdasBatchIma
 // the others: an instance for both spilled 84 bytes and was slower than an integrand
 // kernel and an errors kernel for direct light (two images of 4-D 256x256 and two of
 // 512x512 with 4 spheres: 2.43 ms with two kernels, 2.50 with one instance for both, 2.40
-// with this).
+// with this).  At 64 registers these spill 52 and 20 bytes: the descriptors come from
+// global memory, where the single-image kernels (no spills) have them as parameters; 48
+// registers (5 CTAs per SM) spill 120 and take 2.51 ms.
 template <int D, bool FULL>
 __global__ void __launch_bounds__(256, 4) k_batch_values(const MdasBatchImage* __restrict__ imgs,
                                                       const MdasBatchScene* __restrict__ scenes, int n) {
@@ -390,9 +393,9 @@ __global__ void __launch_bounds__(1024) k_batch_scan(const MdasBatchImage* __res
     scan_image(g, s_sel, s_split, imgs[blockIdx.x].budget, maxPasses);
 }
 
-// ---- adaptive pass: place (one thread per accepted leaf), staged and
-// double-buffered as the single-image kernel: a warp takes 32 consecutive ranks
-// of one image at a time.
+// ---- adaptive pass: place, staged and double-buffered as the single-image kernel: a
+// warp takes 32 consecutive ranks of one image at a time, one accepted leaf per lane.
+// (At D = 4 and 80 registers it spills 12 bytes, which the single-image kernel does not.)
 template <int D>
 __global__ void __launch_bounds__(256, D >= 5 ? 2 : 3) k_batch_place(const MdasBatchImage* __restrict__ imgs, int n) {
     constexpr int CS = RecChunks<D>::CS;

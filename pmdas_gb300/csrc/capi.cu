@@ -1084,7 +1084,9 @@ struct mdas_batch {
     cudaStream_t groupStream[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t forkEvent = nullptr, joinEvent[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaGraphExec_t exec = nullptr;
-    int tune[4] = {4, 4, 4, 8};  // persistent CTAs per SM: errors, decide, place, integrate/integrand
+    // CTAs per SM: initial errors, decide, place, values (and initial sampling,
+    // integrand, integrate)
+    int tune[4] = {4, 4, 4, 8};
     int tileK = MDAS_LEAVES_PER_THREAD;  // leaves per thread of decide (tiles of 256 * tileK leaves)
     uint64_t launches = 0;
     bool anyLearned = false;     // some image takes the learned acceptance

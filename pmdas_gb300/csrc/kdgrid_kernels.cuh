@@ -1200,8 +1200,8 @@ __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.w
 // shared memory at srec (record of lane l at srec + l * CS chunks).
 // Records that are not whole 128-byte lines (D != 4) are fetched in 64-byte pieces:
 // without the hint L2 fetches their neighbours' halves of the shared lines too (5-D
-// 1920x1080 frame at 32 spp 11.56 -> 11.12 ms; with 128- and 256-byte hints 11.56,
-// 12.02 ms; 128-byte records measure the same either way).
+// 1920x1080 frame at 32 spp 12.08 -> 11.63 ms; with a 128-byte hint as without, with a
+// 256-byte one slower; 128-byte records measure the same either way).
 template <int D>
 __device__ __forceinline__ void stage_records(const float* __restrict__ nb, int leaf, float4* srec) {
     constexpr int C = RecChunks<D>::C, CS = RecChunks<D>::CS, NB = NbLayout<D>::FLOATS;

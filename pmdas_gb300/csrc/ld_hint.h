@@ -26,8 +26,9 @@ __device__ __forceinline__ float4 ld4_hint(const float* p) {
     return v;
 }
 
-// The value of sample idx (3 floats at 4-byte alignment), gathered at random from
-// a buffer that the calling kernel does not write.  Without the hint L2 fetches
+// The value of sample idx (3 floats at 4-byte alignment), gathered at random; for words
+// that the calling kernel does not write (read-only loads, and nothing orders them with
+// its stores; it may write other words of the same buffer, as render_sample does).  Without the hint L2 fetches
 // 128 bytes for the 12; with it the errors pass moves a third less DRAM traffic:
 // 87.5 -> 82.3 us per pass on a 4-D 4K frame at 16 spp, 15.5 -> 13.7 us on 4-D
 // 1024x1024, and integrate 4.60 -> 4.50 ms and 0.240 -> 0.237 ms.  Measured and

@@ -338,7 +338,12 @@ int g_sortSpinLimit = 0;
 #ifndef MDAS_SORT_MIN_CTAS
 #define MDAS_SORT_MIN_CTAS 4  // 64 registers: 4 CTAs per SM (the sweep: see kItems)
 #endif
-// One digit position.  Cycles of a CTA's phases decide the order of the steps (5.9 M
+// One digit position, by the chained scan of A. Adinets and D. Merrill ("Onesweep: A
+// Faster Least Significant Digit Radix Sort for GPUs", 2022): one read and one write of
+// the keys, global offsets by look-back (D. Merrill and M. Garland, "Single-pass Parallel
+// Prefix Scan with Decoupled Look-back", 2016).  Ranking a warp's keys through per-digit
+// masks that the lanes OR into shared memory is used by the same family of sorts (CUB's
+// match by atomic OR).  Cycles of a CTA's phases decide the order of the steps (5.9 M
 // keys; 608 CTAs at work at once):
 //   * ranking within the warp was the longest (16 K cycles of 38 K with eight ballots
 //     per row): a row's lanes now leave their bits at their digit in shared memory

@@ -1,5 +1,6 @@
 // shade.cuh — the integrand over the culled disc lists, for every kernel that
-// evaluates samples (the integrand kernels and the render loops' placement).
+// evaluates samples (the integrand kernels, and the values kernels that follow place in
+// the render loops).
 #pragma once
 
 #include "integrand.h"
